@@ -9,16 +9,14 @@
 //   weights  : dW[t][n][c] += sum_p in[p + off(t), c] * g[p, n]
 //
 // Three kernels:
-//   k_conv3x3             forward and data gradient: output channels as the
-//                         MMA's M, 256 (or 128) pixels of one image row as
-//                         its N; input rows TMA-loaded in swizzled layouts,
-//                         the 9 taps as row-shifted descriptors; a ring of
-//                         input rows per column strip (ring mode) or
-//                         three-row stages per tile (step mode, weights
-//                         resident or streamed).
-//   k_conv3x3_wgrad_ring  weight gradient on the same row ring, MN-major,
-//                         accumulators resident in TMEM over each CTA's
-//                         pixel range.
+//   k_conv3x3             forward and data gradient: 128 pixels as the MMA's
+//                         M, output channels as its N; blocks of input rows
+//                         TMA-loaded in swizzled layouts, the 9 taps as
+//                         row-shifted descriptors, weights resident or
+//                         streamed.
+//   k_conv3x3_wgrad_ring  weight gradient on a ring of input rows per column
+//                         strip, MN-major, accumulators resident in TMEM
+//                         over each CTA's pixel range.
 //   k_conv3x3_wgrad       weight gradient for layers whose ring does not fit
 //                         shared memory: (tap, channel) row tiles x output
 //                         channels, pixels split over CTAs, cp.async-staged
@@ -26,6 +24,8 @@
 #include "api_internal.h"
 #include "tc.cuh"
 #include <algorithm>
+#include <cstring>
+#include <utility>
 #include <cudaTypedefs.h>
 #include <type_traits>
 
@@ -34,8 +34,10 @@ namespace {
 
 constexpr int kBM = 128;           // k_conv3x3_wgrad: (tap, c) rows per tile
 constexpr int kThreads = 128;      // k_conv3x3_wgrad
-constexpr int kFwdThreads = 320;  // forward / data gradient: TMA warp, MMA warp, 8 epilogue warps
+constexpr int kFwdThreads = 352;   // k_conv3x3: TMA warp, 2 MMA warps, 8 epilogue warps
+constexpr int kRingThreads = 320;  // k_conv3x3_wgrad_ring: TMA warp, MMA warp, 8 epilogue warps
 constexpr int kMaxStages = 5;
+constexpr int kMaxSlots = 8;       // TMEM accumulators of k_conv3x3
 constexpr int kStages = 4;         // k_conv3x3_wgrad pipeline depth
 constexpr int kWgradBK = 64;       // k_conv3x3_wgrad: pixels per K step
 
@@ -46,12 +48,14 @@ struct ConvArgs {
     float *out_f32;             // [P][N] or null
     int *err;
     int nimg, h, wd, C, N;
-    int KC, RB;                 // channel chunk and its row bytes in shared memory (2 KC, the swizzle span)
-    int NP, MB, M;              // pixels per tile (the MMA's N), 128-row blocks of output channels, MMA M
-    int stages, resident, flip, relu;
-    uint32_t region_bytes;      // one halo row: NP + 2 pixels x RB, rounded up to 1 KB
-    uint32_t wchunk_bytes;      // weights of one channel chunk: [KC / 8][9][N][16 B]
+    int Ng, groups;             // output channels of one CTA and N / Ng
+    int Ws, R, P, TS;           // block: strip width, rows, row pitch Ws + 2, positions between tile starts
+    int KCs, nst, S;            // channels per stage, stages per block (C / KCs), stage buffers
+    int flip, relu, resident;
+    int vec32, vec_f32;         // out and mask 32-byte aligned; out_f32 16-byte aligned
+    uint32_t region_bytes;      // one layout chunk of a stage: (R + 2) P rows, rounded up to 1 KB
     uint32_t stage_bytes, wres_bytes;
+    uint32_t slot_cols, slots;  // TMEM columns per accumulator, accumulators
 };
 
 __device__ __forceinline__ uint32_t tmem_cols(int n) {
@@ -60,98 +64,175 @@ __device__ __forceinline__ uint32_t tmem_cols(int n) {
     return c;
 }
 
-// Forward and data gradient with the output channels on the MMA's M side
-// (M = 64 for up to 64 channels, else 128-row blocks; rows past N read
-// neighbouring weights and their results are never read back) and NP = 256
-// (or 128) pixels of one image row on its N side. One tcgen05.mma costs
-// about the same issue time whatever its shape, so the wide N = 256 tile is
-// what keeps the tensor core busy.
+__device__ __forceinline__ void store32(void *p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+// The epilogue of 16 consecutive channels of one pixel (offset o of the
+// output): bias and ReLU in FP32, then BF16 (times the mask) and / or FP32.
+__device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, const float *bias, size_t o) {
+    float r[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        r[i] = v[i] + bias[i];
+        if (a.relu) r[i] = fmaxf(r[i], 0.f);
+    }
+    if (a.out_f32) {
+        float *dst = a.out_f32 + o;
+        if (a.vec_f32) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<float4 *>(dst + i) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dst[i] = r[i];
+        }
+    }
+    if (!a.out) return;
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(r[2 * i], r[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t *>(&b);
+    }
+    if (a.mask) {
+        const uint4 m0 = __ldg(reinterpret_cast<const uint4 *>(a.mask + o));
+        const uint4 m1 = __ldg(reinterpret_cast<const uint4 *>(a.mask + o) + 1);
+        const uint32_t m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&m[i]));
+            if (!(f.x > 0.f)) w[i] &= 0xffff0000u;
+            if (!(f.y > 0.f)) w[i] &= 0x0000ffffu;
+        }
+    }
+    __nv_bfloat16 *dst = a.out + o;
+    if (a.vec32) {
+        store32(dst, w);
+    } else {
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        *(reinterpret_cast<uint4 *>(dst) + 1) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// Forward and data gradient with 128 pixels on the MMA's M side (one TMEM
+// lane per pixel) and the output channels on its N side: an MMA then costs
+// what its output channels cost and both halves of the array work from 16
+// channels up (the transposed form, channels as M, ran half-empty arrays at
+// 64 channels and a quarter at 32), and the epilogue reads whole pixels, so
+// it needs no transposition. Measured against that form (us): 1920 x 1080
+// 16 -> 32 200 -> 67, 32 -> 32 202 -> 78, 96 -> 32 310 -> 161; 960 x 540
+// 64 -> 64 73 -> 49, 160 -> 64 179 -> 106; 480 x 270 96 -> 96 46 -> 30. The
+// tensor core's operand reads (4 KB + 32 N B of shared memory per MMA, 40
+// cycles at 32 channels, 48 at 64) take about half of the time; the rest is
+// the issue of MMAs and the waits around each tile.
 //
-// A tile is pixels x0 .. x0 + NP - 1 of row y of image b. Per channel chunk
-// of KC a stage holds the three input rows y - 1, y, y + 1, columns
-// x0 - 1 .. x0 + NP, each written by TMA (an NP-wide box and a 2-wide edge
-// box, zero-filled outside the image) in the swizzled K-major layout with
-// RB = 2 KC bytes per pixel row. Tap (dy, dx) is the MMA whose B operand
-// starts dx + 1 rows into row buffer dy + 1: no gather (the swizzle is a
-// function of the absolute shared-memory address, so shifted starts read
-// the rows TMA wrote). The weights (A, [chunk][k group][tap][n][16 B], no
-// swizzle) are loaded by TMA once per CTA when they fit next to the stages,
-// else per stage.
-// Warp roles (no block-wide barrier inside the tile loop):
-//   warp 0     one thread issues the TMA loads of step s into stage s % S
-//              (after the MMAs of step s - S released it) with the bytes
-//              it expects on full[stage].
-//   warp 1     the whole warp runs the MMA loop, one elected lane issues the
-//              step's 9 taps x KC / 16 x MB MMAs into one of two TMEM
-//              accumulator slots and commits them to empty[stage] and,
-//              after a tile's last chunk, to tfull[slot].
-//   warps 2-9  epilogue: TMEM lane quarter warp % 4, half (warp - 2) / 4 of
-//              the tile's pixels; bias / ReLU in FP32, BF16 staged through
-//              shared memory into 16 B stores (ReLU mask applied there).
-//              Then arrive on tempty[slot].
+// A CTA walks blocks of R rows of a strip of Ws columns. A block's input is
+// one TMA box per layout chunk of kc channels, (R + 2) x (Ws + 2) pixels
+// (zero-filled outside the image), which lands as consecutive pixel rows of
+// RB = 2 kc bytes in the swizzled K-major layout with pitch P = Ws + 2
+// pixels. In this flat order tap (dy, dx) of every pixel of the block is
+// the row dy P + dx further on, so an A operand is any 128 consecutive
+// rows: tile t starts at row t TS. With TS = P a tile is one image row
+// (Ws = 128); with TS = 128 the tiles run on across the rows of the block
+// (narrow images and ragged widths), and the two pitch columns per row are
+// computed and dropped. (The swizzle is a function of the absolute
+// shared-memory address, so shifted starts read the rows TMA wrote. The
+// last tile may read past the block: its surplus rows are dropped too.)
+// The channels of a block come in nst stages of KCs channels; with nst > 1
+// all tiles of the block keep their accumulators until the last stage.
+// Weights (B, [layout chunk][tap][n][kc channels], the same swizzled K-major
+// rows, one TMA box per chunk) are loaded once per CTA when they fit next to
+// the stages, else with every stage. (As 16 B rows in the no-swizzle layout
+// the 72 KB of a 64 -> 64 layer took 17 us to load.) Layers whose
+// weights do not fit are split into groups of output channels.
+// Warp roles (no block-wide barrier inside the loop):
+//   warp 0     one thread issues the TMA loads of a stage once the MMAs of
+//              the stage S before it released the buffer.
+//   warps 1-2  issue the MMAs of alternate blocks or tiles; commit to
+//              tfull[slot] after a tile's last stage and to empty[stage].
+//   warps 3-10 epilogue, two groups of four warps taking alternate tiles;
+//              warp % 4 is the TMEM lane quarter (32 pixels). Bias / ReLU in
+//              FP32, 32 B stores.
 // Every wait is bounded and also ends when another role has given up.
-// kKS = KC / 16 (K steps per tap) and kMB are compile-time so that the MMA
-// warp's loop unrolls into base descriptors plus precomputed offsets: the
-// issue loop, not the tensor core, is otherwise the bottleneck.
-template <int kKS, int kMB, bool kRing>
+//
+// The order of the sums is fixed per layer shape (ConvOrder) and does not
+// depend on the tiling: kKK = K steps per channel chunk of the order, kRows:
+// tap rows outside the channel chunks, else the channel chunks outermost.
+template <int kKK, bool kRows>
 __global__ void __launch_bounds__(kFwdThreads, 1)
-    k_conv3x3(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_edge,
-              const __grid_constant__ CUtensorMap map_w, ConvArgs a) {
+    k_conv3x3(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_w, ConvArgs a,
+              int kcl) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], tfull[2], tempty[2], wbar, mma_done;
+    __shared__ uint64_t full[kMaxStages], empty[kMaxStages], tfull[kMaxSlots], tempty[kMaxSlots], wbar, mma_done[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    __shared__ int mma_pace;
-    __shared__ __align__(16) __nv_bfloat16 ostage[8][16 * 32];  // per epilogue warp: 16 pixels x 32 channels
+    __shared__ float s_bias[256];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int KC = 16 * kKS, RB = 2 * KC, KG = KC / 8, MB = kMB;
-    const int C = a.C, N = a.N, W = a.wd, H = a.h, NP = a.NP, S = a.stages;
-    const int chunks = C / KC;
-    const int ntx = (W + NP - 1) / NP, ntiles = a.nimg * H * ntx;
-    const uint32_t region_bytes = a.region_bytes, stage_bytes = a.stage_bytes, wchunk_bytes = a.wchunk_bytes;
-    const uint32_t tap_bytes = (uint32_t)N * 16, wkg_bytes = 9 * tap_bytes;
+    const int N = a.N, Ng = a.Ng, W = a.wd, H = a.h, S = a.S, P = a.P, kc = 1 << kcl, RB = 2 << kcl;
+    const int grp = blockIdx.x % a.groups, ctas = gridDim.x / a.groups, ci = blockIdx.x / a.groups, n0 = grp * Ng;
+    const int ntx = (W + a.Ws - 1) / a.Ws, nrb = (H + a.R - 1) / a.R, nblk = a.nimg * ntx * nrb;
+    const int b_beg = (int)((int64_t)nblk * ci / ctas), b_end = (int)((int64_t)nblk * (ci + 1) / ctas);
+    const uint32_t tap_bytes = (uint32_t)(Ng * RB), wch_bytes = 9 * tap_bytes;  // weights of a tap, of kc channels
     // 1 KB aligned: TMA swizzle atoms and the descriptors' address phase
     unsigned char *const base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     unsigned char *const wres = base;
     unsigned char *const stages = base + a.wres_bytes;
-    const uint32_t slot_cols = (uint32_t)(MB * NP), ncols = tmem_cols(2 * MB * NP);
-    // Step mode: tiles blockIdx.x, + gridDim.x, ... in (image, row, x tile)
-    // order. Ring mode: a contiguous range of tiles in (image, x tile, row)
-    // order, so consecutive tiles are consecutive rows of one column strip.
-    const int t_beg = kRing ? (int)((int64_t)ntiles * blockIdx.x / gridDim.x) : 0;
-    const int my_tiles = kRing ? (int)((int64_t)ntiles * (blockIdx.x + 1) / gridDim.x) - t_beg
-                               : (blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0);
-    auto tile_of = [&](int tl, int &b, int &y, int &x0) {
-        if (kRing) {
-            const int t = t_beg + tl, r2 = t / H;
-            y = t - r2 * H;
-            x0 = (r2 % ntx) * NP;
-            b = r2 / ntx;
-        } else {
-            const int t = blockIdx.x + tl * gridDim.x, by = t / ntx;
-            x0 = (t - by * ntx) * NP;
-            y = by % H;
-            b = by / H;
+    const uint32_t a_bytes = (uint32_t)(a.KCs >> kcl) * a.region_bytes;  // weights of a streamed stage follow
+    const uint32_t ncols = tmem_cols((int)(a.slots * a.slot_cols));
+    // Walks the CTA's blocks (strip by strip, rows downwards) without
+    // divisions, which cost the MMA thread as much as a tile's MMAs.
+    struct Block {
+        int img, y0, x0, rows, w, tiles;
+    };
+    auto fill = [&](Block &k) {
+        k.rows = min(a.R, H - k.y0);
+        k.w = min(a.Ws, W - k.x0);
+        k.tiles = a.TS == P ? k.rows : ((k.rows - 1) * P + k.w + 127) >> 7;
+    };
+    auto first_block = [&]() {
+        Block k;
+        const int r2 = b_beg / nrb;
+        k.y0 = (b_beg - r2 * nrb) * a.R;
+        k.img = r2 / ntx;
+        k.x0 = (r2 - k.img * ntx) * a.Ws;
+        fill(k);
+        return k;
+    };
+    auto next_block = [&](Block &k) {
+        k.y0 += a.R;
+        if (k.y0 >= H) {
+            k.y0 = 0;
+            k.x0 += a.Ws;
+            if (k.x0 >= W) {
+                k.x0 = 0;
+                ++k.img;
+            }
         }
+        fill(k);
     };
     volatile int *abort = &abort_flag;
+    const bool by_tile = a.nst > 1;  // how the two MMA warps share the work
 
     if (tid == 0) {
         for (int i = 0; i < S; ++i) {
             tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
+            tc::mbar_init(&empty[i], by_tile ? 2 : 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < (int)a.slots; ++i) {
             tc::mbar_init(&tfull[i], 1);
-            tc::mbar_init(&tempty[i], 256);
+            tc::mbar_init(&tempty[i], 4);
         }
         tc::mbar_init(&wbar, 1);
-        tc::mbar_init(&mma_done, 1);
+        tc::mbar_init(&mma_done[0], 1);
+        tc::mbar_init(&mma_done[1], 1);
         abort_flag = 0;
-        mma_pace = 0;
         tc::fence_mbar_init();
     }
+    for (int i = tid; i < Ng; i += kFwdThreads) s_bias[i] = a.bias ? a.bias[n0 + i] : 0.f;
     if (warp == 1) tc::tmem_alloc(&tmem_slot, ncols);
     tc::fence_before_sync();
     __syncthreads();
@@ -162,241 +243,209 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         if (lane == 0) {
             // ---- TMA producer ----
             if (a.resident) {
-                tc::mbar_arrive_expect_tx(&wbar, chunks * wchunk_bytes);
-                for (int ch = 0; ch < chunks; ++ch)
-                    for (int kg = 0; kg < KG; ++kg)
-                        tc::tma_load_3d(wres + ch * wchunk_bytes + kg * wkg_bytes, &map_w, ch * KC + kg * 8, 0, 0,
-                                        &wbar);
+                tc::mbar_arrive_expect_tx(&wbar, (uint32_t)(a.C / kc) * wch_bytes);
+                for (int ch = 0; ch < a.C / kc; ++ch)
+                    tc::tma_load_3d(wres + ch * wch_bytes, &map_w, ch * kc, n0, 0, &wbar);
             }
-            int s = 0;
-            if (kRing) {
-                // one row buffer (all channel chunks) per load; a column
-                // strip's first tile loads rows y - 1, y, y + 1, every later
-                // tile only row y + 1
-                const uint32_t tx = (uint32_t)chunks * (NP + 2) * RB;
-                for (int tl = 0; tl < my_tiles && !*abort; ++tl) {
-                    int b, y, x0;
-                    tile_of(tl, b, y, x0);
-                    const bool seg = tl == 0 || y == 0;
-                    bool ok = true;
-                    for (int yy = seg ? y - 1 : y + 1; yy <= y + 1; ++yy, ++s) {
-                        const int st = s % S;
-                        if (s >= S && !tc::mbar_wait_or_abort(&empty[st], ((s / S) - 1) & 1, abort)) {
-                            ok = false;
-                            break;
-                        }
-                        unsigned char *sa = stages + st * stage_bytes;
-                        tc::mbar_arrive_expect_tx(&full[st], tx);
-                        for (int ch = 0; ch < chunks; ++ch) {
-                            tc::tma_load_4d(sa + ch * region_bytes, &map_in, ch * KC, x0 - 1, yy, b, &full[st]);
-                            tc::tma_load_4d(sa + ch * region_bytes + NP * RB, &map_edge, ch * KC, x0 - 1 + NP, yy, b,
-                                            &full[st]);
-                        }
+            const int nch = a.KCs >> kcl;
+            const uint32_t tx = (uint32_t)nch * (uint32_t)((a.R + 2) * P * RB) +
+                                (a.resident ? 0u : (uint32_t)nch * wch_bytes);
+            int buf = 0, issued = -1;
+            uint32_t par = 1;
+            Block k = first_block();
+            for (int b = b_beg; b < b_end && !*abort; ++b, next_block(k)) {
+                bool ok = true;
+                for (int st = 0; st < a.nst; ++st) {
+                    // (a fresh barrier passes a wait for parity 1)
+                    if (!tc::mbar_wait_or_abort(&empty[buf], par, abort)) {
+                        ok = false;
+                        break;
                     }
-                    if (!ok) break;
-                }
-            } else {
-                const uint32_t tx = 3u * (NP + 2) * RB + (a.resident ? 0u : wchunk_bytes);
-                for (int tl = 0; tl < my_tiles && !*abort; ++tl) {
-                    int b, y, x0;
-                    tile_of(tl, b, y, x0);
-                    bool ok = true;
-                    for (int ch = 0; ch < chunks; ++ch, ++s) {
-                        const int st = s % S;
-                        if (s >= S && !tc::mbar_wait_or_abort(&empty[st], ((s / S) - 1) & 1, abort)) {
-                            ok = false;
-                            break;
-                        }
-                        unsigned char *sa = stages + st * stage_bytes;
-                        tc::mbar_arrive_expect_tx(&full[st], tx);
-                        for (int r = 0; r < 3; ++r) {
-                            tc::tma_load_4d(sa + r * region_bytes, &map_in, ch * KC, x0 - 1, y + r - 1, b, &full[st]);
-                            tc::tma_load_4d(sa + r * region_bytes + NP * RB, &map_edge, ch * KC, x0 - 1 + NP,
-                                            y + r - 1, b, &full[st]);
-                        }
-                        if (!a.resident)
-                            for (int kg = 0; kg < KG; ++kg)
-                                tc::tma_load_3d(sa + 3 * region_bytes + kg * wkg_bytes, &map_w, ch * KC + kg * 8, 0, 0,
-                                                &full[st]);
+                    unsigned char *sa = stages + (size_t)buf * a.stage_bytes;
+                    tc::mbar_arrive_expect_tx(&full[buf], tx);
+                    for (int ch = 0; ch < nch; ++ch)
+                        tc::tma_load_4d(sa + ch * a.region_bytes, &map_in, st * a.KCs + ch * kc, k.x0 - 1, k.y0 - 1,
+                                        k.img, &full[buf]);
+                    if (!a.resident)
+                        for (int ch = 0; ch < nch; ++ch)
+                            tc::tma_load_3d(sa + a_bytes + ch * wch_bytes, &map_w, st * a.KCs + ch * kc, n0, 0,
+                                            &full[buf]);
+                    issued = buf > issued ? buf : issued;
+                    if (++buf == S) {
+                        buf = 0;
+                        par ^= 1;
                     }
-                    if (!ok) break;
                 }
+                if (!ok) break;
             }
             // no TMA write may land after the CTA has exited: wait for the
-            // last phase issued on every stage (immediate when consumed)
-            for (int st = 0; st < S && st < s; ++st) {
-                const int last = s - 1 - ((s - 1 - st) % S);
-                tc::mbar_wait(&full[st], (last / S) & 1);
-            }
+            // last phase issued on every stage (immediate when consumed).
+            // par is the parity a buffer's next load would wait for on
+            // empty: from buf on the last load's phase is par, before it the
+            // one after.
+            for (int st = 0; st <= issued; ++st) tc::mbar_wait(&full[st], st < buf ? par ^ 1 : par);
             if (a.resident) tc::mbar_wait(&wbar, 0);
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer: the whole warp runs the loop, one lane issues ----
+    } else if (warp <= 2) {
+        // ---- MMA issuers: one lane of each issues, the control flow is the
+        // whole warp's. Two warps, because the waits and commits around a
+        // tile take a warp as long as a small tile's MMAs take the tensor
+        // core. They take alternate blocks, which keeps them out of step, or
+        // alternate tiles where a block has several stages. ----
         // Descriptor offsets (16 B units in the start-address field, which
-        // never carries: shared addresses stay below 256 KB) of the 9 taps:
-        // B = row buffer r shifted by c rows; A = the tap's weight slice
-        // (mirrored taps for the data gradient).
-        const uint32_t idesc = tc::idesc_bf16(a.M, NP, false, false);
-        uint32_t boff[9], aoff[9];
+        // never carries: shared addresses stay below 256 KB) of the 9 taps
+        // (mirrored weight taps for the data gradient).
+        const uint32_t leader = tc::elect_one() ? 1u : 0u, group = (uint32_t)warp - 1;
+        const uint32_t idesc = tc::idesc_bf16(128, Ng, false, false);
+        uint32_t aoff[9], boff[9];
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
-            const int r = t / 3, c = t % 3, tap = a.flip ? 8 - t : t;
-            boff[t] = (r * region_bytes + c * RB) >> 4;
-            aoff[t] = (tap * tap_bytes) >> 4;
+            aoff[t] = (uint32_t)(((t / 3) * P + t % 3) * RB) >> 4;
+            boff[t] = ((a.flip ? 8 - t : t) * tap_bytes) >> 4;
         }
-        const uint64_t bdesc0 = tc::smem_desc_sw(tc::smem_addr(stages), RB);
-        const uint64_t adesc0 = tc::smem_desc(tc::smem_addr(a.resident ? wres : stages + 3 * region_bytes), wkg_bytes, 128);
-        const uint32_t stage16 = stage_bytes >> 4, wchunk16 = wchunk_bytes >> 4, kstep_a16 = (2 * wkg_bytes) >> 4;
-        int s = 0;
-        bool run = !a.resident || tc::mbar_wait_or_abort_warp(&wbar, 0, abort);
-        if (kRing) {
-            // rows top, top + 1, top + 2 of the load sequence; after the
-            // tile, row `top` is released (all three at a strip's end)
-            int top = 0;
-            for (int tl = 0; tl < my_tiles && run; ++tl) {
-                int b, y, x0;
-                tile_of(tl, b, y, x0);
-                if (tl == 0 || y == 0) {
-                    top = s;
-                    s += 3;
-                } else {
-                    top += 1;
-                    s += 1;
+        const uint64_t adesc0 = tc::smem_desc_sw(tc::smem_addr(stages), RB);
+        const uint64_t bdesc0 = tc::smem_desc_sw(tc::smem_addr(a.resident ? wres : stages + a_bytes), RB);
+        const uint32_t stage16 = a.stage_bytes >> 4, region16 = a.region_bytes >> 4;
+        const uint32_t wch16 = wch_bytes >> 4, ts16 = (uint32_t)(a.TS * RB) >> 4;
+        constexpr int KCo = 16 * kKK;
+        const int subs = a.KCs / KCo;
+        auto wait = [&](uint64_t *bar, uint32_t parity) {
+            return __all_sync(0xffffffffu, tc::mbar_ready(bar, parity)) ||
+                   tc::mbar_wait_or_abort_warp(bar, parity, abort);
+        };
+        int buf = 0;  // stage buffer and the parity of its next phase
+        uint32_t buf_par = 0;
+        // the block's first tile, its accumulator and the parity of that
+        // accumulator's release (a fresh barrier passes a wait for parity 1)
+        uint32_t slot0 = 0, par0 = 1;
+        const uint32_t tstep = by_tile ? 2 : 1;
+        bool run = !a.resident || wait(&wbar, 0);
+        Block k = first_block();
+        for (int b = b_beg; b < b_end && run; ++b, next_block(k)) {
+            const uint32_t tiles = (uint32_t)k.tiles;
+            const bool mine = by_tile || ((uint32_t)(b - b_beg) & 1) == group;
+            // by tiles: the tiles whose accumulator has this warp's parity
+            const uint32_t first = by_tile ? (slot0 ^ group) & 1 : 0;
+            for (int st = 0; st < a.nst && run && mine; ++st) {
+                if (!wait(&full[buf], buf_par)) {
+                    run = false;
+                    break;
                 }
-                const int slot = tl & 1;
-                if (tl >= 2 && !tc::mbar_wait_or_abort_warp(&tempty[slot], ((tl >> 1) - 1) & 1, abort)) break;
                 tc::fence_after_sync();
-                const uint32_t d = tmem + slot * slot_cols;
-                for (int r = 0; r < 3 && run; ++r) {
-                    const int ld = top + r, st = ld % S;
-                    if (!tc::mbar_wait_or_abort_warp(&full[st], (ld / S) & 1, abort)) {
-                        run = false;
-                        break;
+                uint64_t ad = adesc0 + buf * stage16 + first * ts16;
+                const uint64_t bd_stage =
+                    bdesc0 + (a.resident ? (uint32_t)(st * (a.KCs >> kcl)) * wch16 : buf * stage16);
+                uint32_t slot = slot0 + first, par = par0;
+                for (uint32_t t = first; t < tiles; t += tstep, ad += tstep * ts16, slot += tstep) {
+                    if (slot >= a.slots) {
+                        slot -= a.slots;
+                        par ^= 1;
                     }
-                    tc::fence_after_sync();
-                    const uint64_t bd = bdesc0 + st * stage16;
-                    for (int ch = 0; ch < chunks; ++ch) {
-                        const uint64_t bdc = bd + ((ch * region_bytes) >> 4);
-                        const uint64_t adc = adesc0 + ch * wchunk16;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-#pragma unroll
-                            for (int kk = 0; kk < kKS; ++kk)
-#pragma unroll
-                                for (int mb = 0; mb < kMB; ++mb)
-                                    tc::mma_bf16_warp(d + mb * NP, adc + aoff[3 * r + c] + kk * kstep_a16 + mb * 128,
-                                                      bdc + ((c * RB) >> 4) + kk * 2, idesc,
-                                                      r > 0 || ch > 0 || c > 0 || kk > 0);
+                    if (st == 0) {
+                        if (!wait(&tempty[slot], par)) {
+                            run = false;
+                            break;
+                        }
+                        tc::fence_after_sync();
                     }
-                    // A shared-memory atomic by the issuing lane after each
-                    // row of MMAs. Measured on B200: without it the kernel
-                    // takes 2.3x as long (0.56 against 0.24 ms at 1920x1080,
-                    // 64 -> 64); a plain store, a tcgen05 fence, a sleep of
-                    // up to 60 ns or a spinning test_wait do not help.
-                    if (lane == 0) atomicAdd(&mma_pace, 1);
-                }
-                if (!run) break;
-                const bool strip_ends = tl + 1 == my_tiles || y + 1 == H;
-                for (int r = 0; r < (strip_ends ? 3 : 1); ++r) tc::mma_commit_warp(tc::smem_addr(&empty[(top + r) % S]));
-                tc::mma_commit_warp(tc::smem_addr(&tfull[slot]));
-            }
-        } else {
-            for (int tl = 0; tl < my_tiles && run; ++tl) {
-                const int slot = tl & 1;
-                if (tl >= 2 && !tc::mbar_wait_or_abort_warp(&tempty[slot], ((tl >> 1) - 1) & 1, abort)) break;
-                tc::fence_after_sync();
-                const uint32_t d = tmem + slot * slot_cols;
-                for (int ch = 0; ch < chunks; ++ch, ++s) {
-                    const int st = s % S;
-                    if (!tc::mbar_wait_or_abort_warp(&full[st], (s / S) & 1, abort)) {
-                        run = false;
-                        break;
-                    }
-                    tc::fence_after_sync();
-                    const uint64_t bd = bdesc0 + st * stage16;
-                    const uint64_t ad = adesc0 + (a.resident ? ch * wchunk16 : st * stage16);
+                    const uint32_t d = tmem + slot * a.slot_cols;
+                    if (kRows) {
+                        // rows of taps, channel chunks, columns of taps
 #pragma unroll
-                    for (int t = 0; t < 9; ++t)
+                        for (int r = 0; r < 3; ++r)
+                            for (int ch = 0; ch < subs; ++ch) {
+                                const uint64_t adc = ad + ch * region16;
+                                const uint64_t bdc = bd_stage + (uint32_t)ch * wch16;
 #pragma unroll
-                        for (int kk = 0; kk < kKS; ++kk)
+                                for (int c = 0; c < 3; ++c)
 #pragma unroll
-                            for (int mb = 0; mb < kMB; ++mb)
-                                tc::mma_bf16_warp(d + mb * NP, ad + aoff[t] + kk * kstep_a16 + mb * 128, bd + boff[t] + kk * 2,
-                                                  idesc, ch > 0 || t > 0 || kk > 0);
-                    if (lane == 0) atomicAdd(&mma_pace, 1);  // see the ring-mode loop
-                    tc::mma_commit_warp(tc::smem_addr(&empty[st]));
-                    if (ch == chunks - 1) tc::mma_commit_warp(tc::smem_addr(&tfull[slot]));
-                }
-            }
-        }
-        // every MMA issued has finished before TMEM is released
-        tc::mma_commit_warp(tc::smem_addr(&mma_done));
-        if (lane == 0) tc::mbar_wait(&mma_done, 0);
-        __syncwarp();
-    } else {
-        // ---- epilogue ----
-        // TMEM lane quarter q holds channels q * cpq .. + cpq - 1 of each
-        // 128-row block in its first cpq lanes (M = 128: 32 per quarter;
-        // M = 64: rows 16 q .. 16 q + 15 sit in lanes 32 q .. 32 q + 15).
-        // Per 16-pixel chunk the warp converts its channels to BF16 (bias,
-        // ReLU), stages them as [pixel][channel] in shared memory and writes
-        // 16 B pieces (8 channels of one pixel; the ReLU mask applied there).
-        const int q = warp & 3, half = (warp - 2) >> 2;
-        const int cpq = a.M == 64 ? 16 : 32, pieces = 16 * cpq / 8;
-        const int cbeg = half * (NP / 2), cend = cbeg + NP / 2;
-        __nv_bfloat16 *const os = ostage[warp - 2];
-        for (int tl = 0; tl < my_tiles; ++tl) {
-            const int slot = tl & 1;
-            if (!tc::mbar_wait_or_abort(&tfull[slot], (tl >> 1) & 1, abort)) break;
-            tc::fence_after_sync();
-            int b, y, x0;
-            tile_of(tl, b, y, x0);
-            const size_t row_pix = ((size_t)b * H + y) * W;
-            for (int mb = 0; mb < MB; ++mb) {
-                const int cq = mb * 128 + q * cpq;  // first channel of this quarter
-                if (cq >= N) continue;             // warp-uniform: no channels here
-                const int co = cq + lane;
-                const bool cvalid = lane < cpq && co < N;
-                const float bias = (a.bias && cvalid) ? a.bias[co] : 0.f;
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + slot * slot_cols + mb * NP;
-                for (int col = cbeg; col < cend && x0 + col < W; col += 16) {
-                    float v[16];
-                    tc::tmem_ld16(taddr + col, v);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        v[i] += bias;
-                        if (a.relu) v[i] = fmaxf(v[i], 0.f);
-                    }
-                    if (a.out_f32 && cvalid)
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (x0 + col + i < W) a.out_f32[(row_pix + x0 + col + i) * N + co] = v[i];
-                    if (!a.out) continue;
-                    if (lane < cpq)
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) os[i * cpq + lane] = __float2bfloat16_rn(v[i]);
-                    __syncwarp();
-                    for (int j = lane; j < pieces; j += 32) {
-                        const int px = j / (cpq / 8), part = j - px * (cpq / 8);
-                        const int c8 = cq + part * 8;
-                        if (x0 + col + px < W && c8 < N) {
-                            uint4 val = *reinterpret_cast<const uint4 *>(os + px * cpq + part * 8);
-                            const size_t o = (row_pix + x0 + col + px) * N + c8;
-                            if (a.mask) {
-                                const uint4 mv = *reinterpret_cast<const uint4 *>(a.mask + o);
-                                const __nv_bfloat16 *mb16 = reinterpret_cast<const __nv_bfloat16 *>(&mv);
-                                __nv_bfloat16 *vb = reinterpret_cast<__nv_bfloat16 *>(&val);
-                                for (int e = 0; e < 8; ++e)
-                                    if (!(__bfloat162float(mb16[e]) > 0.f)) vb[e] = __float2bfloat16_rn(0.f);
+                                    for (int kk = 0; kk < kKK; ++kk)
+                                        tc::mma_bf16_pred(leader, d, adc + aoff[3 * r + c] + kk * 2,
+                                                          bdc + boff[3 * r + c] + kk * 2, idesc,
+                                                          st > 0 || r > 0 || ch > 0 || c > 0 || kk > 0);
                             }
-                            *reinterpret_cast<uint4 *>(a.out + o) = val;
+                    } else {
+                        for (int ch = 0; ch < subs; ++ch) {
+                            const int co = ch * KCo;
+                            const uint32_t chunk = (uint32_t)co >> kcl, in_chunk = (uint32_t)(co & (kc - 1)) >> 3;
+                            const uint64_t adc = ad + chunk * region16 + in_chunk;
+                            const uint64_t bdc = bd_stage + chunk * wch16 + in_chunk;
+#pragma unroll
+                            for (int tp = 0; tp < 9; ++tp)
+#pragma unroll
+                                for (int kk = 0; kk < kKK; ++kk)
+                                    tc::mma_bf16_pred(leader, d, adc + aoff[tp] + kk * 2,
+                                                      bdc + boff[tp] + kk * 2, idesc,
+                                                      st > 0 || ch > 0 || tp > 0 || kk > 0);
                         }
                     }
-                    __syncwarp();
+                    if (st == a.nst - 1) tc::mma_commit_pred(leader, tc::smem_addr(&tfull[slot]));
+                }
+                tc::mma_commit_pred(leader, tc::smem_addr(&empty[buf]));
+                if (++buf == S) {
+                    buf = 0;
+                    buf_par ^= 1;
                 }
             }
-            tc::fence_before_sync();
-            tc::mbar_arrive(&tempty[slot]);  // this slot's TMEM reads are done
+            if (!mine && ++buf == S) {  // (one stage per block)
+                buf = 0;
+                buf_par ^= 1;
+            }
+            for (slot0 += tiles; slot0 >= a.slots; slot0 -= a.slots) par0 ^= 1;
+        }
+        // every MMA issued has finished before TMEM is released
+        tc::mma_commit_pred(leader, tc::smem_addr(&mma_done[group]));
+        wait(&mma_done[group], 0);
+    } else {
+        // ---- epilogue: one thread per pixel of the tile ----
+        const int q = warp & 3;
+        const uint32_t group = (uint32_t)(warp - 3) >> 2;
+        uint32_t slot = group, par = 0, mine = group;  // mine = 0: the next tile is this group's
+        bool run = true;
+        Block k = first_block();
+        for (int b = b_beg; b < b_end && run; ++b, next_block(k)) {
+            for (int t = 0; t < k.tiles; ++t) {
+                if (mine) {
+                    mine = 0;
+                    continue;
+                }
+                mine = 1;
+                if (!tc::mbar_wait_or_abort(&tfull[slot], par, abort)) {
+                    run = false;
+                    break;
+                }
+                __syncwarp();
+                tc::fence_after_sync();
+                const int pos = t * a.TS + q * 32 + lane;
+                const int row = pos / P, col = pos - row * P;
+                const bool valid = row < k.rows && col < k.w;
+                const size_t o = (((size_t)k.img * H + k.y0 + row) * W + k.x0 + col) * N + n0;
+                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + slot * a.slot_cols;
+                for (int c = 0; c < Ng; c += 32) {
+                    float v[32];
+                    __syncwarp();
+                    if (c + 32 <= Ng) {
+                        tc::tmem_ld32(taddr + c, v);
+                    } else {
+                        float h16[16];
+                        tc::tmem_ld16(taddr + c, h16);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = h16[i];
+                    }
+                    if (valid) {
+                        conv_store16(a, v, s_bias + c, o + c);
+                        if (c + 32 <= Ng) conv_store16(a, v + 16, s_bias + c + 16, o + c + 16);
+                    }
+                }
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&tempty[slot]);  // this quarter's TMEM reads are done
+                slot += 2;  // an even number of accumulators
+                if (slot >= a.slots) {
+                    slot -= a.slots;
+                    par ^= 1;
+                }
+            }
         }
     }
     tc::fence_before_sync();
@@ -432,7 +481,7 @@ struct WgradRingArgs {
 };
 
 template <int kKS, int kGS>  // input chunk KC = 16 kKS, gradient channel group 16 kGS
-__global__ void __launch_bounds__(kFwdThreads, 1)
+__global__ void __launch_bounds__(kRingThreads, 1)
     k_conv3x3_wgrad_ring(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_edge,
                          const __grid_constant__ CUtensorMap map_g, WgradRingArgs a) {
     extern __shared__ unsigned char smem_raw[];
@@ -765,6 +814,135 @@ void encode_map(CUtensorMap *m, const void *ptr, cuuint32_t rank, const cuuint64
 
 size_t round1k(size_t v) { return (v + 1023) & ~(size_t)1023; }
 
+// The order in which a layer sums its products, a function of its shape
+// only: the MMAs of one output run over channel chunks of KCo channels (all
+// nine taps of a chunk, then the next chunk) or, with rows_outer, over the
+// three tap rows with the chunks inside. BF16 activations round the sums,
+// so a different order would flip roundings layer by layer; the thresholds
+// below keep every shape's order, and with it every output bit, as it was
+// under the tiling they came from (channels as M, 256 pixels as N).
+struct ConvOrder {
+    int KCo;
+    bool rows_outer;
+};
+
+ConvOrder conv_order(int C, int N, int w) {
+    const int np = (N > 128 || w <= 128) ? 128 : 256;
+    const size_t cap = 220 * 1024 - 1024 - 2048 - 8192, wbytes = round1k((size_t)9 * N * C * 2);
+    auto region = [&](int rb) { return round1k((size_t)(np + 2) * rb); };
+    const int kc = C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16;
+    if (wbytes + 4 * (C / kc) * region(2 * kc) <= cap) return {kc, C > kc};
+    for (int c : {64, 32, 16})
+        if (C % c == 0 && wbytes + 9 * region(2 * c) <= cap) return {c, false};
+    for (int ns : {4, 3, 2})
+        for (int c : {64, 32, 16})
+            if ((ns >= 3 || c == 16) && C % c == 0 && ns * (3 * region(2 * c) + round1k((size_t)c * 18 * N)) <= cap)
+                return {c, false};
+    throw Error(CRT_ERR_INVALID, "conv3x3: tile does not fit shared memory");
+}
+
+// The tiling of a layer, by a cost model in SM cycles: an MMA of 128 x Ng
+// x 16 reads 4 KB + 32 Ng B of shared memory at 128 B per cycle or
+// multiplies at 4096 MAC per cycle, whichever is longer; a CTA's loads run
+// at about 32 B per cycle; an epilogue group needs about 400 + 10 Ng cycles
+// per tile and there are two; an MMA warp needs about 58 cycles per MMA and
+// 250-300 per tile, and there are two. A block takes the longest of these,
+// and the layer the CTA with the most blocks.
+struct ConvPlan {
+    int Ng, groups, Ws, R, TS, KCs, kc, S, resident, grid;
+    double cost;
+};
+
+// Rows of shared memory that a block's last tile reads past its stage
+// (their results are dropped).
+size_t conv_over_rows(int tiles, int TS, int R, int P) { return (size_t)std::max(0, (tiles - 1) * TS + 130 - R * P); }
+
+ConvPlan conv_plan(const ConvOrder &ord, int nimg, int h, int w, int C, int N, int sms) {
+    ConvPlan best{};
+    best.cost = 1e30;
+    const size_t cap = 227 * 1024 - 1024 - 4096;  // minus base alignment and static shared memory
+    for (int groups = 1; groups <= N / 16; ++groups) {
+        if (N % (16 * groups)) continue;
+        const int Ng = N / groups;
+        const size_t wall = (size_t)18 * Ng * C;
+        int stride = 32;
+        while (stride < Ng) stride <<= 1;
+        const int slots = std::min(kMaxSlots, 512 / stride);
+        const double mma = 9.0 * (C / 16) * std::max(0.5 * Ng, 34.0 + 0.25 * Ng);
+        const double epi = 0.5 * (400.0 + 10.0 * Ng);
+        for (int KCs : {C, 64, 32, 16}) {
+            if (KCs > C || C % KCs || KCs % ord.KCo || (ord.rows_outer && KCs != C)) continue;
+            const int kc = KCs % 64 == 0 ? 64 : KCs % 32 == 0 ? 32 : 16;
+            const int nst = C / KCs;
+            for (int resident = 1; resident >= 0; --resident) {
+                if (resident && wall > cap) continue;
+                if (!resident && KCs > 64) continue;
+                for (int mode = 0; mode < 3; ++mode) {
+                    // one image row of 128 pixels per tile, or tiles across
+                    // the rows of strips of equal width (at most 254; at
+                    // most 126 for shorter blocks)
+                    const int lim = mode == 1 ? 254 : 126;
+                    const int strips = mode == 0 ? (w + 127) / 128 : (w + lim - 1) / lim;
+                    const int Ws = mode == 0 ? 128 : (w + strips - 1) / strips;
+                    const int P = Ws + 2, TS = mode == 0 ? P : 128;
+                    for (int R : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
+                        if (R > h && R > 1) break;
+                        const int tiles = mode == 0 ? R : ((R - 1) * P + Ws + 127) / 128;
+                        if (nst > 1 && tiles > slots) break;
+                        const size_t region = round1k((size_t)(R + 2) * P * 2 * kc);
+                        const size_t stage = (KCs / kc) * region + (resident ? 0 : round1k((size_t)18 * Ng * KCs));
+                        const size_t fixed = (resident ? round1k(wall) : 0) + conv_over_rows(tiles, TS, R, P) * 2 * kc;
+                        if (fixed + stage > cap) break;
+                        const int S = (int)std::min<size_t>(kMaxStages, (cap - fixed) / stage);
+                        const int64_t nblk = (int64_t)nimg * strips * ((h + R - 1) / R);
+                        const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(nblk, sms / groups));
+                        const int64_t rounds = (nblk + ctas - 1) / ctas;
+                        const double load = ((double)(R + 2) * P * 2 * C + (resident ? 0.0 : (double)wall)) / 32;
+                        double total;
+                        if (nst == 1) {  // the warps take alternate blocks
+                            const double issue = tiles * (9.0 * (C / 16) * 58 + 300) + 400;
+                            const double pipe = std::max(std::max(tiles * mma, load), tiles * epi);
+                            total = S > 1 || rounds == 1 ? std::max(rounds * pipe, (rounds + 1) / 2 * issue)
+                                                         : rounds * (issue + load + 1000);
+                        } else {  // alternate tiles of each stage
+                            const double issue = (tiles + 1) / 2 * (9.0 * (KCs / 16) * 58 + 250) + 350;
+                            const double stage_t = std::max(std::max(tiles * mma / nst, load / nst), issue);
+                            total = rounds * std::max(nst * (S > 1 ? stage_t : stage_t + load / nst + 1000), tiles * epi);
+                        }
+                        const double cost = total + load / nst + 2 * epi + (resident ? wall / 40.0 : 0.0);
+                        if (cost < best.cost)
+                            best = ConvPlan{Ng, groups, Ws, R, TS, KCs, kc, S, resident, ctas * groups, cost};
+                    }
+                }
+            }
+        }
+    }
+    CRT_CHECK(best.cost < 1e30, CRT_ERR_INVALID, "conv3x3: tile does not fit shared memory");
+    return best;
+}
+
+// The order and plan of a shape: the search takes a few microseconds, more
+// than a launch, so each thread keeps the last few dozen shapes' results.
+std::pair<ConvOrder, ConvPlan> conv_lookup(int nimg, int h, int w, int C, int N) {
+    struct Entry {
+        int key[6];
+        ConvOrder ord;
+        ConvPlan plan;
+    };
+    thread_local Entry cache[64] = {};
+    const int key[6] = {nimg, h, w, C, N, sm_count()};
+    uint32_t hash = 2166136261u;
+    for (int k : key) hash = (hash ^ (uint32_t)k) * 16777619u;
+    Entry &e = cache[(hash >> 16 ^ hash) & 63];
+    if (std::memcmp(e.key, key, sizeof(key)) != 0) {
+        const ConvOrder ord = conv_order(C, N, w);
+        e.plan = conv_plan(ord, nimg, h, w, C, N, key[5]);
+        e.ord = ord;
+        std::memcpy(e.key, key, sizeof(key));
+    }
+    return {e.ord, e.plan};
+}
+
 }  // namespace
 
 void conv3x3_check(int C, int N) {
@@ -787,6 +965,7 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
                   (!out_f32 || (reinterpret_cast<uintptr_t>(out_f32) & 3) == 0) &&
                   (!mask || (reinterpret_cast<uintptr_t>(mask) & 15) == 0),
               CRT_ERR_INVALID, "conv3x3: output and mask must be 16-byte aligned");
+    const auto [ord, pl] = conv_lookup(nimg, h, w, C, N);
     ConvArgs a;
     a.bias = bias;
     a.mask = mask;
@@ -798,93 +977,52 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
     a.wd = w;
     a.C = C;
     a.N = N;
+    a.Ng = pl.Ng;
+    a.groups = pl.groups;
+    a.Ws = pl.Ws;
+    a.R = pl.R;
+    a.P = pl.Ws + 2;
+    a.TS = pl.TS;
+    a.KCs = pl.KCs;
+    a.nst = C / pl.KCs;
+    a.S = pl.S;
     a.flip = flip ? 1 : 0;
     a.relu = relu ? 1 : 0;
-    // Tile: 256 pixels (one MMA of N = 256) unless the image is at most 128
-    // wide or there are more than 128 output channels (two 128-row M
-    // blocks; the TMEM then holds 2 slots x 2 x 128 columns).
-    a.MB = N > 128 ? 2 : 1;
-    a.M = N <= 64 ? 64 : 128;  // M = 64 spreads the channels over all four TMEM lane quarters
-    a.NP = (a.MB == 2 || w <= 128) ? 128 : 256;
-    const size_t kCap = 220 * 1024 - 1024 - 2048 - 8192;  // minus base alignment, over-read pad, epilogue staging
-    const size_t wbytes = round1k((size_t)9 * N * C * 2);
-    auto region = [&](int rb) { return round1k((size_t)(a.NP + 2) * rb); };
-    a.KC = 0;
-    a.stages = 0;
-    a.resident = 0;
-    bool ring = false;
-    // Ring mode (preferred): resident weights and a ring of 4 or 5 input
-    // rows, each holding all channels in chunks of the widest KC dividing C;
-    // every input row is then loaded once per column strip.
-    {
-        const int kc = C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16;
-        const size_t row = (size_t)(C / kc) * region(2 * kc);
-        for (int ns : {5, 4})
-            if (!a.KC && wbytes + ns * row <= kCap) {
-                a.KC = kc;
-                a.stages = ns;
-                a.resident = 1;
-                ring = true;
-            }
-    }
-    // Step mode: a stage is one channel chunk of the three rows of one tile.
-    // Row bytes RB = 2 KC of 128, 64 or 32 (the TMA swizzle span); weights
-    // resident when they fit next to at least 3 stages (widest chunk first,
-    // then the deepest pipeline), else streamed with every stage.
-    for (int rb : {128, 64, 32})
-        for (int ns : {5, 4, 3})
-            if (!a.KC && C % (rb / 2) == 0 && wbytes + ns * 3 * region(rb) <= kCap) {
-                a.KC = rb / 2;
-                a.stages = ns;
-                a.resident = 1;
-            }
-    // (a pipeline of 3 or 4 stages at any chunk width first: the streamed
-    // weights dominate a stage; two stages only for the widest layers)
-    for (int ns : {4, 3, 2})
-        for (int rb : {128, 64, 32})
-            if (!a.KC && (ns >= 3 || rb == 32) && C % (rb / 2) == 0 &&
-                ns * (3 * region(rb) + round1k((size_t)(rb / 16) * 9 * N * 16)) <= kCap) {
-                a.KC = rb / 2;
-                a.stages = ns;
-            }
-    CRT_CHECK(a.KC > 0, CRT_ERR_INVALID, "conv3x3: tile does not fit shared memory");
-    a.RB = 2 * a.KC;
-    a.region_bytes = (uint32_t)region(a.RB);
-    a.wchunk_bytes = (uint32_t)((a.KC / 8) * 9 * N * 16);
-    a.stage_bytes = (uint32_t)(ring ? (size_t)(C / a.KC) * a.region_bytes
-                                    : 3 * a.region_bytes + (a.resident ? 0 : round1k(a.wchunk_bytes)));
-    a.wres_bytes = a.resident ? (uint32_t)round1k((size_t)(C / a.KC) * a.wchunk_bytes) : 0u;
-    const size_t smem = 1024 + a.wres_bytes + (size_t)a.stages * a.stage_bytes + 2048;
+    a.resident = pl.resident;
+    a.vec32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+    a.vec_f32 = (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0;
+    const int RB = 2 * pl.kc;
+    a.region_bytes = (uint32_t)round1k((size_t)(a.R + 2) * a.P * RB);
+    a.stage_bytes = (uint32_t)((a.KCs / pl.kc) * a.region_bytes +
+                               (a.resident ? 0 : round1k((size_t)18 * a.Ng * a.KCs)));
+    a.wres_bytes = a.resident ? (uint32_t)round1k((size_t)18 * a.Ng * C) : 0u;
+    a.slot_cols = 32;
+    while ((int)a.slot_cols < a.Ng) a.slot_cols <<= 1;
+    a.slots = std::min<uint32_t>(kMaxSlots, 512 / a.slot_cols);
+    const int tiles = a.TS == a.P ? a.R : ((a.R - 1) * a.P + a.Ws + 127) / 128;
+    const size_t smem =
+        1024 + a.wres_bytes + (size_t)a.S * a.stage_bytes + conv_over_rows(tiles, a.TS, a.R, a.P) * RB;
 
     // input [nimg][h][w][C] as 4D (C, w, h, nimg); weights [9][N][C] as 3D (C, N, 9)
-    CUtensorMap map_in, map_edge, map_w;
-    const CUtensorMapSwizzle swz = a.RB == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                                   : a.RB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                                : CU_TENSOR_MAP_SWIZZLE_32B;
+    CUtensorMap map_in, map_w;
+    const CUtensorMapSwizzle swz = RB == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                   : RB == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                              : CU_TENSOR_MAP_SWIZZLE_32B;
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)nimg};
     const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)w * C * 2, (cuuint64_t)h * w * C * 2};
-    const cuuint32_t box[4] = {(cuuint32_t)a.KC, (cuuint32_t)a.NP, 1, 1};
-    const cuuint32_t box_edge[4] = {(cuuint32_t)a.KC, 2, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)pl.kc, (cuuint32_t)a.P, (cuuint32_t)(a.R + 2), 1};
     encode_map(&map_in, in, 4, dims, strides, box, swz);
-    encode_map(&map_edge, in, 4, dims, strides, box_edge, swz);
     const cuuint64_t wdims[3] = {(cuuint64_t)C, (cuuint64_t)N, 9};
     const cuuint64_t wstrides[2] = {(cuuint64_t)C * 2, (cuuint64_t)N * C * 2};
-    const cuuint32_t wbox[3] = {8, (cuuint32_t)N, 9};
-    encode_map(&map_w, wgt, 3, wdims, wstrides, wbox, CU_TENSOR_MAP_SWIZZLE_NONE);
+    const cuuint32_t wbox[3] = {(cuuint32_t)pl.kc, (cuuint32_t)a.Ng, 9};
+    encode_map(&map_w, wgt, 3, wdims, wstrides, wbox, swz);
 
-    using Kfn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, ConvArgs);
-    const Kfn kfns[2][2][3] = {{{k_conv3x3<1, 1, false>, k_conv3x3<2, 1, false>, k_conv3x3<4, 1, false>},
-                                {k_conv3x3<1, 2, false>, k_conv3x3<2, 2, false>, k_conv3x3<4, 2, false>}},
-                               {{k_conv3x3<1, 1, true>, k_conv3x3<2, 1, true>, k_conv3x3<4, 1, true>},
-                                {k_conv3x3<1, 2, true>, k_conv3x3<2, 2, true>, k_conv3x3<4, 2, true>}}};
-    const Kfn kfn = kfns[ring ? 1 : 0][a.MB - 1][a.KC == 16 ? 0 : a.KC == 32 ? 1 : 2];
+    using Kfn = void (*)(CUtensorMap, CUtensorMap, ConvArgs, int);
+    const Kfn kfns[2][3] = {{k_conv3x3<1, false>, k_conv3x3<2, false>, k_conv3x3<4, false>},
+                            {k_conv3x3<1, true>, k_conv3x3<2, true>, k_conv3x3<4, true>}};
+    const Kfn kfn = kfns[ord.rows_outer ? 1 : 0][ord.KCo == 16 ? 0 : ord.KCo == 32 ? 1 : 2];
     CRT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    CRT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kFwdThreads, smem));
-    per_sm = std::max(1, std::min(per_sm, 512 / host_tmem_cols(2 * a.MB * a.NP)));
-    const int64_t tiles = (int64_t)nimg * h * ((w + a.NP - 1) / a.NP);
-    const int grid = (int)std::min<int64_t>(tiles, (int64_t)sm_count() * per_sm);
-    kfn<<<grid, kFwdThreads, smem, s>>>(map_in, map_edge, map_w, a);
+    kfn<<<pl.grid, kFwdThreads, smem, s>>>(map_in, map_w, a, pl.kc == 64 ? 6 : pl.kc == 32 ? 5 : 4);
     CRT_CUDA(cudaGetLastError());
 }
 
@@ -948,7 +1086,7 @@ bool wgrad_ring_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *d
     CRT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t tiles = (int64_t)nimg * h * ((w + a.NP - 1) / a.NP);
     const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count() / a.G > 0 ? sm_count() / a.G : 1));
-    kfn<<<ctas * a.G, kFwdThreads, smem, s>>>(map_in, map_edge, map_g, a);
+    kfn<<<ctas * a.G, kRingThreads, smem, s>>>(map_in, map_edge, map_g, a);
     CRT_CUDA(cudaGetLastError());
     return true;
 }
