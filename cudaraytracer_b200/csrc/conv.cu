@@ -34,8 +34,7 @@ namespace {
 
 constexpr int kBM = 128;           // k_conv3x3_wgrad: (tap, c) rows per tile
 constexpr int kThreads = 128;      // k_conv3x3_wgrad
-constexpr int kFwdThreads = 352;   // k_conv3x3: TMA warp, 2 MMA warps, 8 epilogue warps
-constexpr int kRingThreads = 320;  // k_conv3x3_wgrad_ring: TMA warp, MMA warp, 8 epilogue warps
+constexpr int kConvThreads = 352;  // k_conv3x3, k_conv3x3_wgrad_ring: TMA warp, 2 MMA warps, 8 epilogue warps
 constexpr int kMaxStages = 5;
 constexpr int kMaxSlots = 8;       // TMEM accumulators of k_conv3x3
 constexpr int kStages = 4;         // k_conv3x3_wgrad pipeline depth
@@ -162,7 +161,7 @@ __device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, 
 // depend on the tiling: kKK = K steps per channel chunk of the order, kRows:
 // tap rows outside the channel chunks, else the channel chunks outermost.
 template <int kKK, bool kRows>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+__global__ void __launch_bounds__(kConvThreads, 1)
     k_conv3x3(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_w, ConvArgs a,
               int kcl) {
     extern __shared__ unsigned char smem_raw[];
@@ -232,7 +231,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         abort_flag = 0;
         tc::fence_mbar_init();
     }
-    for (int i = tid; i < Ng; i += kFwdThreads) s_bias[i] = a.bias ? a.bias[n0 + i] : 0.f;
+    for (int i = tid; i < Ng; i += kConvThreads) s_bias[i] = a.bias ? a.bias[n0 + i] : 0.f;
     if (warp == 1) tc::tmem_alloc(&tmem_slot, ncols);
     tc::fence_before_sync();
     __syncthreads();
@@ -470,6 +469,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // channels, TMA-loaded, MN-major). Blocks of one CTA group: TMEM holds
 // (blocks per group) x N columns; with more blocks than fit, the grid is
 // split into groups that each accumulate a subset and read all inputs.
+// Bound by the MMAs' issue and, for small batches, by the start-up and the
+// atomics of the epilogue. One issuing lane per warp in a warp-uniform loop,
+// two issuing warps and the rotated epilogue against one warp with an
+// elect.sync per MMA (us): 960 x 540 64 x 64 86 -> 56, 1920 x 1080 32 x 32
+// 214 -> 143, 8 x 64 x 64 160 x 64 47 -> 34, 8 x 128 x 128 32 x 32 27 -> 21.
 struct WgradRingArgs {
     float *dw;  // [9][N][C], accumulated
     int *err;
@@ -481,13 +485,13 @@ struct WgradRingArgs {
 };
 
 template <int kKS, int kGS>  // input chunk KC = 16 kKS, gradient channel group 16 kGS
-__global__ void __launch_bounds__(kRingThreads, 1)
+__global__ void __launch_bounds__(kConvThreads, 1)
     k_conv3x3_wgrad_ring(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_edge,
                          const __grid_constant__ CUtensorMap map_g, WgradRingArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint64_t full[kMaxStages], empty[kMaxStages], gfull[2], gempty[2], mma_done;
     __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag, mma_pace;
+    __shared__ int abort_flag;
     constexpr int KC = 16 * kKS, RB = 2 * KC, GKC = 16 * kGS, RBG = 2 * GKC;
     constexpr int TPB = KC == 64 ? 2 : 3;  // valid taps (dx) per 128-row block
     constexpr int BPD = KC == 64 ? 2 : 1;  // blocks per (input row, channel chunk)
@@ -515,15 +519,14 @@ __global__ void __launch_bounds__(kRingThreads, 1)
     if (tid == 0) {
         for (int i = 0; i < S; ++i) {
             tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
+            tc::mbar_init(&empty[i], 2);
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(&gfull[i], 1);
-            tc::mbar_init(&gempty[i], 1);
+            tc::mbar_init(&gempty[i], 2);
         }
-        tc::mbar_init(&mma_done, 1);
+        tc::mbar_init(&mma_done, 2);
         abort_flag = 0;
-        mma_pace = 0;
         tc::fence_mbar_init();
     }
     if (warp == 1) tc::tmem_alloc(&tmem_slot, ncols);
@@ -574,8 +577,11 @@ __global__ void __launch_bounds__(kRingThreads, 1)
             }
             for (int t2 = tl > 2 ? tl - 2 : 0; t2 < tl; ++t2) tc::mbar_wait(&gfull[t2 & 1], (t2 >> 1) & 1);
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer (whole warp, one elected lane issues) ----
+    } else if (warp <= 2) {
+        // ---- MMA issuers: one lane of each issues, the control flow is the
+        // whole warp's; the two warps take alternate blocks ----
+        const uint32_t leader = tc::elect_one() ? 1u : 0u;
+        const int group = warp - 1;
         const uint32_t idesc = tc::idesc_bf16(128, N, true, true);
         const uint32_t ring_addr = tc::smem_addr(ring), gbuf_addr = tc::smem_addr(gbuf);
         const int ksteps = NP / 16;
@@ -606,29 +612,30 @@ __global__ void __launch_bounds__(kRingThreads, 1)
 #pragma unroll
                     for (int bb = 0; bb < BPD; ++bb) {
                         const int blk = (ri * chunks + ch) * BPD + bb;
-                        if (blk < b_beg || blk >= b_end) continue;
+                        if (blk < b_beg || blk >= b_end || (blk & 1) != group) continue;
                         const uint32_t d = tmem + (uint32_t)(blk - b_beg) * N;
                         const uint64_t ad0 = tc::smem_desc_sw(
                             ring_addr + st * a.row_bytes + ch * a.region_bytes + bb * TPB * RB, RB, RB);
                         for (int kk = 0; kk < ksteps; ++kk)
-                            tc::mma_bf16_warp(d, ad0 + ((kk * 16 * RB) >> 4), bd0 + ((kk * 16 * RBG) >> 4), idesc,
+                            tc::mma_bf16_pred(leader, d, ad0 + ((kk * 16 * RB) >> 4), bd0 + ((kk * 16 * RBG) >> 4), idesc,
                                               tl > 0 || kk > 0);
                     }
-                if (lane == 0) atomicAdd(&mma_pace, 1);  // see k_conv3x3's ring loop
             }
             if (!run) break;
             const bool strip_ends = tl + 1 == my_tiles || y + 1 == H;
-            for (int r = 0; r < (strip_ends ? 3 : 1); ++r) tc::mma_commit_warp(tc::smem_addr(&empty[(top + r) % S]));
-            tc::mma_commit_warp(tc::smem_addr(&gempty[gs]));
+            for (int r = 0; r < (strip_ends ? 3 : 1); ++r) tc::mma_commit_pred(leader, tc::smem_addr(&empty[(top + r) % S]));
+            tc::mma_commit_pred(leader, tc::smem_addr(&gempty[gs]));
         }
-        tc::mma_commit_warp(tc::smem_addr(&mma_done));
-        if (lane == 0) tc::mbar_wait(&mma_done, 0);
-        __syncwarp();
+        tc::mma_commit_pred(leader, tc::smem_addr(&mma_done));
+        tc::mbar_wait_or_abort_warp(&mma_done, 0, abort);
     } else {
         // ---- epilogue: add the accumulators into dW ----
-        const int q = warp & 3, half = (warp - 2) >> 2, r = q * 32 + lane;
+        const int q = warp & 3, half = (warp - 3) >> 2, r = q * 32 + lane;
         const bool ok = tc::mbar_wait_or_abort(&mma_done, 0, abort);
         tc::fence_after_sync();
+        // All CTAs add into the same 9 N C sums at about the same time: each
+        // starts at columns of its own.
+        const int rot = (ci * 16) % N;
         if (ok && my_tiles > 0 && !*abort)
             for (int blk = b_beg + half; blk < b_end; blk += 2) {
                 const int bb = blk % BPD, rc = blk / BPD, ch = rc % chunks, ri = rc / chunks;
@@ -636,8 +643,10 @@ __global__ void __launch_bounds__(kRingThreads, 1)
                 const bool valid = r / KC < TPB && gtap < 3;
                 const int t = ri * 3 + gtap;
                 const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(blk - b_beg) * N;
-                for (int n0 = 0; n0 < N; n0 += 16) {
+                for (int nr = 0; nr < N; nr += 16) {
+                    const int n0 = nr + rot < N ? nr + rot : nr + rot - N;
                     float v[16];
+                    __syncwarp();
                     tc::tmem_ld16(taddr + n0, v);
                     if (valid)
 #pragma unroll
@@ -1022,7 +1031,7 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
                             {k_conv3x3<1, true>, k_conv3x3<2, true>, k_conv3x3<4, true>}};
     const Kfn kfn = kfns[ord.rows_outer ? 1 : 0][ord.KCo == 16 ? 0 : ord.KCo == 32 ? 1 : 2];
     CRT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kfn<<<pl.grid, kFwdThreads, smem, s>>>(map_in, map_w, a, pl.kc == 64 ? 6 : pl.kc == 32 ? 5 : 4);
+    kfn<<<pl.grid, kConvThreads, smem, s>>>(map_in, map_w, a, pl.kc == 64 ? 6 : pl.kc == 32 ? 5 : 4);
     CRT_CUDA(cudaGetLastError());
 }
 
@@ -1086,7 +1095,7 @@ bool wgrad_ring_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *d
     CRT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t tiles = (int64_t)nimg * h * ((w + a.NP - 1) / a.NP);
     const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, sm_count() / a.G > 0 ? sm_count() / a.G : 1));
-    kfn<<<ctas * a.G, kRingThreads, smem, s>>>(map_in, map_edge, map_g, a);
+    kfn<<<ctas * a.G, kConvThreads, smem, s>>>(map_in, map_edge, map_g, a);
     CRT_CUDA(cudaGetLastError());
     return true;
 }

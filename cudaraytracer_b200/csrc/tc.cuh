@@ -82,33 +82,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         : "memory");
 }
 
-// The same, executed by a whole converged warp: one lane (elect.sync)
-// issues. Running the issue loop warp-uniformly lets the compiler keep the
-// descriptors in uniform registers; a loop under `if (lane == 0)` pays
-// register moves per MMA and issues far slower.
-__device__ __forceinline__ void mma_bf16_warp(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              bool accumulate) {
-    const uint32_t acc = accumulate ? 1u : 0u, z = 0u;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(z), "r"(z), "r"(z), "r"(z)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit_warp(uint32_t mbar) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred e;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
-        "}\n" ::"r"(mbar)
-        : "memory");
-}
-
 // The same with the issuing lane chosen by the caller (`leader` non-zero in
 // one lane, the same lane for a whole accumulation and its commit): the
 // loop stays warp-uniform without an elect.sync per MMA.
@@ -256,8 +229,8 @@ __device__ __forceinline__ bool elect_one() {
 
 // Warp-uniform form of mbar_wait_or_abort: every lane polls and the warp
 // leaves together. (With one lane polling for the others, the warp could
-// stay split after the wait; every elect.sync of an MMA loop then waits for
-// the other part, 300 instead of 55 cycles per MMA.)
+// stay split after the wait, and an MMA loop with an elect.sync per MMA then
+// took 300 instead of 55 cycles per MMA.)
 __device__ __forceinline__ bool mbar_wait_or_abort_warp(uint64_t *bar, uint32_t parity, volatile int *abort) {
     for (int round = 0; round < 256; ++round) {
         if (__any_sync(0xffffffffu, *abort != 0)) return false;
