@@ -35,6 +35,7 @@ __global__ void k_raygen_views(const CamView *cams, int n_views, StepParams sp, 
         counters[kHitCounter] = 0;
         counters[kMissCounter] = 0;
         counters[kSssCounter] = 0;
+        counters[kPathCounter] = 0;
     }
     if (i >= n) return;
     const int64_t g = base + i;
@@ -109,6 +110,7 @@ int render_views(Scene &sc, const std::vector<CameraState> &cams, int first_samp
     const int smem = sc.rp.traversal(sc.bvh.num_tris);
     const int g_sh = persistent_grid((const void *)k_shade, blk);
     const int g_sm = persistent_grid((const void *)k_shade_miss, blk);
+    const int b_paths = path_start(smem, chunk);
     StepParams sp;
     sp.bounce = 0;
     sp.rr = sc.rp.rr;
@@ -123,6 +125,10 @@ int render_views(Scene &sc, const std::vector<CameraState> &cams, int first_samp
             const int in = b & 1, out = 1 - in;
             StepParams bp = sp;
             bp.bounce = b;
+            if (b >= b_paths) {
+                launch_paths(view, bp, sc.rp.max_bounces, chunk, q[in], sc.wf.counters + in, sc.wf.counters, av, s);
+                break;
+            }
             launch_extend_stage(view.bvh, q[in], sc.wf.counters + in, sc.wf.hits, sc.wf.counters, out, smem, b,
                                 ord, blk, s);
             k_shade<<<g_sh, blk, 0, s>>>(view, bp, q[in], sc.wf.hits, sc.wf.counters + in, q[out], sc.wf.counters,

@@ -18,6 +18,8 @@
 // Rows are bottom-up (pixel j = 0 is the bottom row), as the reference's
 // accumulation buffers.
 #include "path.cuh"
+#include "path_loop.cuh"
+#include "tiny.cuh"
 #include "traverse.cuh"
 #include <algorithm>
 #include <cmath>
@@ -379,6 +381,7 @@ __global__ void k_raygen(CamView cam, StepParams sp, int n, QueueView q, int *co
         counters[kHitCounter] = 0;
         counters[kMissCounter] = 0;
         counters[kSssCounter] = 0;
+        counters[kPathCounter] = 0;
     }
     if (i >= n) return;
     uint32_t pixel = (uint32_t)(i % sp.pixels);
@@ -709,6 +712,77 @@ void launch_shadow_stage(const BvhView &bvh, const ShadowView &sh, int *counters
                                                                                    term1, acc, mode);
 }
 
+// The rest of every path of a queue in one kernel (path_loop.cuh), over the
+// tree in global or (kTiny) in shared memory.
+template <bool kTiny>
+struct SceneSrc {
+    static constexpr bool kTraceLast = true;
+    const SceneView &s;
+    const StepParams &sp;
+    const QueueView &q;
+    const AccumView &acc;
+    int limit;
+    const float4 *tree;  // kTiny: interior nodes, then triangle records
+    __device__ bool load(int i, PathState &ps, int &max_bounces) {
+        ps = load_path(q, i);
+        max_bounces = limit;
+        return true;
+    }
+    __device__ const SceneView &scene() { return s; }
+    __device__ StepParams params() { return sp; }
+    template <bool kEarlyExit>
+    __device__ Hit trace(V3 o, V3 d, float tmin, float tmax, float t_exit) {
+        LocalStack st;
+        if (kTiny)
+            return closest_hit_tiny<kEarlyExit>(tree, tree + 4 * s.bvh.num_nodes, s.bvh, st, o, d, tmin, tmax, t_exit);
+        return closest_hit_st<kEarlyExit, true, false>(s.bvh, st, o, d, tmin, tmax, t_exit);
+    }
+    __device__ Hit closest(V3 o, V3 d) { return trace<false>(o, d, 0.f, kTriTMax, 0.f); }
+    __device__ bool visible(const NeeRecord &nee) {
+        ShadowRay r;
+        shadow_ray_init(r, nee.hp, nee.hn, nee.lp, nee.ln);
+        return shadow_ray_visible(r, s.bvh, trace<true>(r.o, r.dir, 1e-6f, 1e8f, r.t_exit));
+    }
+    __device__ void add(const PathState &ps) { accumulate(acc, ps.pixel, ps.dc, ps.ic); }
+};
+
+// Compiled for two register budgets. With 3 resident blocks per SM (168
+// registers) a small pass finishes sooner; with 8 (64 registers, as the shade
+// stage) a large one has the warps to cover instruction fetch (Cornell box,
+// 262,144 / 8,388,608 paths: 610 / 11,205 us with 3, 690 / 10,507 us with 8).
+template <bool kTiny, int kMinBlocks>
+__global__ void __launch_bounds__(kPathBlock, kMinBlocks) k_paths(SceneView s, StepParams sp, int max_bounces,
+                                                                  QueueView q, const int *n_in, int *counters,
+                                                                  AccumView acc) {
+    extern __shared__ float4 s_tree[];
+    if (kTiny) {
+        tiny_fill(s_tree, s.bvh);
+        __syncthreads();
+    }
+    SceneSrc<kTiny> src{s, sp, q, acc, max_bounces, s_tree};
+    const uint2 rays = path_loop(src, *n_in, sp.bounce, counters + kPathCounter);
+    const unsigned e = __reduce_add_sync(0xffffffffu, rays.x), v = __reduce_add_sync(0xffffffffu, rays.y);
+    if ((threadIdx.x & 31) == 0) {
+        if (e) atomicAdd(reinterpret_cast<unsigned long long *>(counters + kExtendRaysCounter), (unsigned long long)e);
+        if (v) atomicAdd(reinterpret_cast<unsigned long long *>(counters + kShadowRaysCounter), (unsigned long long)v);
+    }
+}
+
+int path_start(int mode, int n) {
+    if (mode != kStageLocal && mode != kStageRefill) return INT_MAX;
+    return n <= kPathFromStart ? 0 : n <= kPathFromSecond ? 1 : 2;
+}
+
+void launch_paths(const SceneView &view, const StepParams &sp, int max_bounces, int n, const QueueView &q,
+                  const int *n_in, int *counters, const AccumView &acc, cudaStream_t s) {
+    const int64_t tb = tiny_bytes(view.bvh);
+    const bool tiny = tb <= kTinyDefaultBytes, few = n <= kPathFewPaths;
+    const auto kernel = tiny ? (few ? k_paths<true, 3> : k_paths<true, 8>)
+                             : (few ? k_paths<false, 3> : k_paths<false, 8>);
+    kernel<<<persistent_grid((const void *)kernel, kPathBlock), kPathBlock, tiny ? (size_t)tb : 0, s>>>(
+        view, sp, max_bounces, q, n_in, counters, acc);
+}
+
 // The mode named by CRT_STAGE_TRAVERSAL, or -1.
 static int env_traversal() {
     const char *e = getenv("CRT_STAGE_TRAVERSAL");
@@ -797,9 +871,15 @@ int render_samples(const SceneView &view, const CameraState &cam, const RenderPa
         sp.pixels = pixels;
         k_raygen<<<(n + 255) / 256, 256, 0, stream>>>(cv, sp, n, q[0], wf.counters);
         ++launches;
+        const int b_paths = path_start(smem, n);
         for (int b = 0; b < rp.max_bounces; ++b) {
             int in = b & 1, out = 1 - in;
             sp.bounce = b;
+            if (b >= b_paths) {
+                launch_paths(view, sp, rp.max_bounces, n, q[in], wf.counters + in, wf.counters, av, stream);
+                ++launches;
+                break;
+            }
             launch_extend_stage(view.bvh, q[in], wf.counters + in, wf.hits, wf.counters, out, smem, b, ord, blk,
                                 stream);
             if (mb == 4)

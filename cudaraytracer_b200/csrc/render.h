@@ -58,6 +58,7 @@ constexpr int kWavefrontCounters = 16;
 constexpr int kHitCounter = 4;
 constexpr int kMissCounter = 5;
 constexpr int kSssCounter = 6;
+constexpr int kPathCounter = 7;  // paths the path kernel has handed out
 constexpr int kExtendRaysCounter = 8;
 constexpr int kShadowRaysCounter = 10;
 

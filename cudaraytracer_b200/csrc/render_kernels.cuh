@@ -78,6 +78,27 @@ void launch_extend_stage(const BvhView &bvh, const QueueView &q, const int *n_in
 void launch_shadow_stage(const BvhView &bvh, const ShadowView &sh, int *counters, const QueueView &qout,
                          float4 *term0, float4 *term1, const AccumView &acc, int mode, int block, cudaStream_t s);
 
+// The path kernel (path_loop.cuh): every path of queue q (count *n_in) from
+// bounce sp.bounce to its end; raygen has reset counters[kPathCounter].
+// path_start is the bounce from which a pass of n paths in stage-traversal
+// mode `mode` goes to it (INT_MAX: never): a stage costs its slowest warp's
+// latency and three more launches, 17 us with no path left in it and 65 us
+// with a few, so late bounces and small passes belong in one kernel, while
+// the first bounces of large passes run better as stages (compaction, full
+// warps, 64-register shade). Measured, us per pass, stages only / path
+// kernel from bounce 0 / 1 / 2, at 65,536, 1,048,576 and 8,388,608 paths:
+// Cornell box 696/340/376/392, 1734/1668/1610/1596, 10723/10757/10420/10507;
+// one 1,280-triangle sphere 507/103/164/217, 1022/988/639/718,
+// 4365/7535/3942/4036; the 1.31M-triangle field 1101/310/491/668,
+// 1882/1251/1130/1236, 4987/6512/5194/4349.
+constexpr int kPathBlock = 128;
+constexpr int kPathFromStart = 640 << 10;   // largest pass for the path kernel alone
+constexpr int kPathFromSecond = 2560 << 10; // largest pass for it from bounce 1
+constexpr int kPathFewPaths = 400 << 10;    // largest pass for its large register budget
+int path_start(int mode, int n);
+void launch_paths(const SceneView &view, const StepParams &sp, int max_bounces, int n, const QueueView &q,
+                  const int *n_in, int *counters, const AccumView &acc, cudaStream_t s);
+
 // Blocks per grid for a persistent launch of `kernel` (all SMs at full
 // occupancy).
 int persistent_grid(const void *kernel, int block);

@@ -137,9 +137,14 @@ extern "C" crt_status crt_render_device_noalloc(crt_scene *scene, int32_t first_
             sp.first_sample = first_sample + done;
             sp.pixels = (int)pixels;
             k_raygen<<<(n + 255) / 256, 256, 0, s>>>(cv, sp, n, q[0], counters);
+            const int b_paths = path_start(smem, n);
             for (int b = 0; b < rp.max_bounces; ++b) {
                 const int in = b & 1, out = 1 - in;
                 sp.bounce = b;
+                if (b >= b_paths) {
+                    launch_paths(view, sp, rp.max_bounces, n, q[in], counters + in, counters, av, s);
+                    break;
+                }
                 launch_extend_stage(view.bvh, q[in], counters + in, hits, counters, out, smem, b, ord, blk, s);
                 k_shade<<<g_sh, blk, 0, s>>>(view, sp, q[in], hits, counters + in, q[out], counters, out, sh, term0,
                                             term1, av, ord);

@@ -208,7 +208,10 @@ typedef struct crt_render_params {
 } crt_render_params;
 
 /* crt_render_params.stage_traversal: where each path's traversal stack lives
- * and which node layout it reads. */
+ * and which node layout it reads. With DEFAULT, LOCAL and REFILL the late
+ * bounces of a pass, and all bounces of a small one, run in one kernel that
+ * keeps a path per lane (local stack, float nodes); the others keep the
+ * stage kernels throughout. */
 #define CRT_STAGE_DEFAULT 0       /* CRT_STAGE_TRAVERSAL from the environment, else LOCAL */
 #define CRT_STAGE_LOCAL 1         /* 64-entry stack in local memory, 64 B float nodes */
 #define CRT_STAGE_SHARED 2        /* top 8 entries in shared memory, 64 B float nodes */
