@@ -47,6 +47,7 @@ struct BvhView {
     int *err;              // device error word (kErrTraversalBounds), or null
     const float4 *cnodes;  // the binary nodes with 16-bit quantised boxes, 2 float4 each (bvh16.cuh)
     QuantGrid grid;
+    const float4 *flat;    // scenes of at most kFlatTris triangles: 4 float4 per triangle and the scales (flat.cuh)
 };
 
 #ifdef __CUDACC__

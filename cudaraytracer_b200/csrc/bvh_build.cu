@@ -18,6 +18,7 @@
 // Min/max reductions are order-independent and all partitions are stable, so
 // the tree (and thus tie-breaking between equal-t triangles) is reproducible.
 #include "bvh_build.h"
+#include "flat.cuh"
 #include <vector>
 #include <algorithm>
 #include <cstring>
@@ -684,6 +685,41 @@ struct DevBuf {
 
 }  // namespace
 
+// The records of a scene of at most kFlatTris triangles (flat.cuh), leaf
+// order, one thread per triangle, and the scales after them.
+__global__ void k_flat(const float4 *tris, int n, float4 *flat) {
+    __shared__ float s_e[kFlatTris], s_v[kFlatTris];
+    const int k = threadIdx.x;
+    if (k < n) {
+        const float4 a = tris[3 * k], b = tris[3 * k + 1], c = tris[3 * k + 2];
+        const V3 v0 = v3(a.x, a.y, a.z), e1 = vsub(v3(b.x, b.y, b.z), v0), e2 = vsub(v3(c.x, c.y, c.z), v0);
+        const V3 nn = vcross(e2, e1), f1 = vcross(e1, v0), f2 = vcross(e2, v0);
+        // component j of triangle k: float 2 j + k % 2 of its pair
+        const float r[16] = {nn.x, nn.y, nn.z, vdot(v0, nn), e2.x, e2.y, e2.z, f2.x,
+                             e1.x, e1.y, e1.z, f2.y,         f1.x, f1.y, f1.z, f2.z};
+        float *p = reinterpret_cast<float *>(flat) + 32 * (k / 2) + (k & 1);
+        for (int j = 0; j < 16; ++j) p[2 * j] = r[j];
+        // an odd scene's last record has no second triangle: T = -1 there
+        // (det = 0 and a zero v0 would leave it a candidate)
+        if (k == n - 1 && !(k & 1))
+            for (int j = 0; j < 16; ++j) p[2 * j + 1] = j == 3 ? -1e30f : 0.f;
+        s_e[k] = fmaxf(fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z), fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z));
+        s_v[k] = fabsf(v0.x) + fabsf(v0.y) + fabsf(v0.z);
+    }
+    __syncthreads();
+    if (k == 0) {
+        float e = 0.f, v = 0.f;
+        for (int i = 0; i < n; ++i) {
+            e = fmaxf(e, s_e[i]);
+            v = fmaxf(v, s_v[i]);
+        }
+        // NaN vertices must not pass for small ones
+        for (int i = 0; i < n; ++i)
+            if (!(s_e[i] <= e) || !(s_v[i] <= v)) e = v = INFINITY;
+        flat[8 * ((n + 1) / 2)] = make_float4(e, v, 0.f, 0.f);
+    }
+}
+
 void build_bvh(const float *d_verts, int n, cudaStream_t stream, BvhBuffers &out) {
     CRT_CHECK(n > 0, CRT_ERR_INVALID, "scene has no triangles");
     CRT_CHECK(n < (1 << 27) - 1, CRT_ERR_CAPACITY, "more than 2^27-2 triangles");
@@ -818,6 +854,11 @@ void build_bvh(const float *d_verts, int n, cudaStream_t stream, BvhBuffers &out
     out.num_tris = n;
     // the 16-bit quantised copy of the nodes (bvh16.cuh), one kernel
     build_bvh16(out, out.err, stream);
+    if (n <= kFlatTris) {
+        CRT_CUDA(cudaMalloc(&out.flat, (size_t)flat_float4s(n) * sizeof(float4)));
+        k_flat<<<1, kFlatTris, 0, stream>>>(out.tris, n, out.flat);
+        CRT_CUDA(cudaGetLastError());
+    }
     CRT_CUDA(cudaStreamSynchronize(stream));
     // The 8-wide quantised tree is built only on request (CRT_BVH8=1): its
     // traversal measured slower than the binary one on the icosphere field.
@@ -836,6 +877,7 @@ void free_bvh(BvhBuffers &b) {
     if (b.wnodes) cudaFree(b.wnodes);
     if (b.wlinks) cudaFree(b.wlinks);
     if (b.cnodes) cudaFree(b.cnodes);
+    if (b.flat) cudaFree(b.flat);
     b = BvhBuffers();
 }
 

@@ -25,8 +25,9 @@ struct BvhBuffers {
     int *err = nullptr;  // the owning context's device error word
     float4 *cnodes = nullptr;  // 16-bit quantised copy of `nodes` (bvh16.cuh)
     QuantGrid grid{};
+    float4 *flat = nullptr;    // records of a small scene (flat.cuh), else null
     BvhView view() const {
-        return BvhView{nodes, tris, num_tris, wnodes, wlinks, (int)num_nodes, err, cnodes, grid};
+        return BvhView{nodes, tris, num_tris, wnodes, wlinks, (int)num_nodes, err, cnodes, grid, flat};
     }
 };
 

@@ -20,6 +20,7 @@
 // order of the float atomics that add paths into its pixels.
 #include "api_internal.h"
 #include "path.cuh"
+#include "path_loop.cuh"
 #include <algorithm>
 #include <deque>
 #include <map>
@@ -58,6 +59,7 @@ __global__ void ks_raygen(const ReqDesc *reqs, const Segment *segs, int nseg, in
         counters[kHitCounter] = 0;
         counters[kMissCounter] = 0;
         counters[kSssCounter] = 0;
+        counters[kPathCounter] = 0;
     }
     if (i >= n) return;
     int lo = 0, hi = nseg - 1;
@@ -261,6 +263,51 @@ __global__ void __launch_bounds__(128) ks_shadow(const SceneView *scenes, const 
     }
 }
 
+// The rest of every path of a pass in one kernel (path_loop.cuh), each lane
+// with its path's scene and request; register budgets as k_paths (render.cu).
+struct ServeSrc {
+    static constexpr bool kTraceLast = false;
+    const SceneView *scenes;
+    const ReqDesc *reqs;
+    const QueueView &q;
+    const SceneView *s;
+    const ReqDesc *r;
+    __device__ bool load(int i, PathState &ps, int &max_bounces) {
+        ps = load_path(q, i);
+        const uint32_t tag = path_tag(q, i);
+        s = scenes + (tag >> kSlotBits);
+        r = reqs + (tag & kSlotMask);
+        max_bounces = r->max_bounces;
+        return true;
+    }
+    __device__ const SceneView &scene() { return *s; }
+    __device__ StepParams params() {
+        StepParams sp;
+        sp.rr = r->rr;
+        sp.rr_start = r->rr_start;
+        return sp;
+    }
+    __device__ Hit closest(V3 o, V3 d) {
+        const BvhView bvh = s->bvh;
+        return closest_hit<false>(bvh, o, d, 0.f, kTriTMax);
+    }
+    __device__ bool visible(const NeeRecord &nee) {
+        const BvhView bvh = s->bvh;
+        return crt::visible(bvh, nee.hp, nee.hn, nee.lp, nee.ln);
+    }
+    __device__ void add(const PathState &ps) {
+        accumulate(AccumView{r->direct, r->indirect, nullptr}, ps.pixel, ps.dc, ps.ic);
+    }
+};
+
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kPathBlock, kMinBlocks) ks_paths(const SceneView *scenes, const ReqDesc *reqs,
+                                                                   int bounce, QueueView q, const int *n_in,
+                                                                   int *counters) {
+    ServeSrc src{scenes, reqs, q, scenes, reqs};
+    path_loop(src, *n_in, bounce, counters + kPathCounter);
+}
+
 size_t scene_device_bytes(const Scene &sc) {
     const size_t n = (size_t)sc.bvh.num_tris;
     size_t b = (size_t)sc.bvh.num_nodes * 64 + n * 48 + n * 4;  // nodes, leaf-order triangles, slot_of_prim
@@ -321,7 +368,7 @@ struct crt_server {
     std::multimap<size_t, float4 *> pool;  // released accumulator buffers by size
     size_t bytes_scenes = 0, bytes_wavefront = 0, bytes_requests = 0, bytes_pool = 0;
     int64_t n_running = 0, n_done = 0;
-    int g_ext = 0, g_sh = 0, g_sm = 0, g_sd = 0;
+    int g_ext = 0, g_sh = 0, g_sm = 0, g_sd = 0, g_few = 0, g_many = 0;
 
     ~crt_server() {
         if (stream) cudaStreamSynchronize(stream);
@@ -458,8 +505,18 @@ struct crt_server {
         const ShadeOrder ord{wf.order, (int)wf.cap, nullptr};  // ks_extend takes each path's scene's classes
         ks_raygen<<<(n + 255) / 256, 256, 0, stream>>>(d_reqs, ds, nseg, n, q[0], wf.counters);
         const int smem = stage_traversal_env();
+        const int b_paths = path_start(smem, n);
         for (int b = 0; b < max_b; ++b) {
             const int in = b & 1, out = 1 - in;
+            if (b >= b_paths) {
+                if (n <= kPathFewPaths)
+                    ks_paths<3><<<g_few, kPathBlock, 0, stream>>>(d_scenes, d_reqs, b, q[in], wf.counters + in,
+                                                                   wf.counters);
+                else
+                    ks_paths<8><<<g_many, kPathBlock, 0, stream>>>(d_scenes, d_reqs, b, q[in], wf.counters + in,
+                                                                    wf.counters);
+                break;
+            }
             ks_extend<<<g_ext, 128, 0, stream>>>(d_scenes, q[in], wf.counters + in, wf.hits, wf.counters, out, smem,
                                                  ord);
             ks_shade<<<g_sh, 128, 0, stream>>>(d_scenes, d_reqs, b, q[in], wf.hits, wf.counters + in, q[out],
@@ -532,6 +589,8 @@ extern "C" crt_status crt_server_create(crt_ctx *ctx, const crt_server_config *c
         s->g_sh = persistent_grid((const void *)ks_shade, 128);
         s->g_sm = persistent_grid((const void *)ks_shade_miss, 128);
         s->g_sd = persistent_grid((const void *)ks_shadow, 128);
+        s->g_few = persistent_grid((const void *)ks_paths<3>, kPathBlock);
+        s->g_many = persistent_grid((const void *)ks_paths<8>, kPathBlock);
         *out = s.release();
     });
 }

@@ -8,6 +8,7 @@
 #include "trace.cuh"
 #include "traverse.cuh"
 #include "tiny.cuh"
+#include "flat.cuh"
 #include "render_kernels.cuh"  // persistent_grid
 #include <algorithm>
 #include <cstdlib>
@@ -213,6 +214,21 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_tiny(Job job, int n) {
     }
 }
 
+// One ray per thread over the scene's triangles (flat.cuh).
+template <class Job, bool kEarlyExit>
+__global__ void __launch_bounds__(kTraceBlock) k_trace_flat(Job job, int n) {
+    __shared__ float4 rec[kFlatWords];
+    flat_fill(rec, job.bvh);
+    __syncthreads();
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    BvhView b;
+    V3 o, d;
+    float tmin, tmax, t_exit;
+    job.setup((int)r, b, o, d, tmin, tmax, t_exit);
+    job.finish((int)r, b, closest_hit_flat<kEarlyExit>(rec, job.bvh, o, d, tmin, tmax, t_exit));
+}
+
 // Launches k_trace_tiny over n rays: one ray per thread (persistent false)
 // or a grid of all SMs at full occupancy.
 template <class Job, bool kEarlyExit, int kShort>
@@ -337,8 +353,9 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
     trace_dynamic8<true, kShort, ShadowJob, true>(job, n, s_stack);
 }
 
-// Traversal variant of the trace kernels. The default is kTinyVariant for
-// scenes of at most kTinyDefaultBytes and kTraceVariant otherwise;
+// Traversal variant of the trace kernels. The default is kFlatVariant for
+// scenes of at most kFlatTris triangles, kTinyVariant for others of at most
+// kTinyDefaultBytes and kTraceVariant otherwise;
 // CRT_TRAVERSAL overrides it.
 //   2        binary tree, stack in local memory, per-lane refill;
 //   210/212  the same capped at 51 / 42 registers (10 / 12 blocks per SM);
@@ -356,6 +373,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
 //            kTinyBytes, else 2): one ray per thread with the local stack /
 //            a persistent grid / one ray per thread with 8 stack entries
 //            per lane in shared memory.
+//   14       every triangle, no tree (k_trace_flat; scenes of at most
+//            kFlatTris triangles, else 2): the default there.
 // On the Cornell box (36 triangles, 1M random rays) 11 issues from 85% of
 // the scheduler slots with 11-12 of 32 lanes active: divergence between the
 // lanes' paths, not memory, bounds it. Capping it at 40 / 32 registers (12 /
@@ -363,12 +382,14 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
 // octant before tracing them, measured 8-20% and 2-10% slower.
 constexpr int kTraceVariant = 2;
 constexpr int kTinyVariant = 11;
+constexpr int kFlatVariant = 14;
 
 static int traversal_variant(const BvhView &bvh) {
     const char *e = getenv("CRT_TRAVERSAL");
     const int64_t tb = tiny_bytes(bvh);
     const bool tiny = tb <= kTinyBytes;
-    int v = e ? atoi(e) : (tb <= kTinyDefaultBytes ? kTinyVariant : kTraceVariant);
+    int v = e ? atoi(e) : bvh.flat ? kFlatVariant : (tb <= kTinyDefaultBytes ? kTinyVariant : kTraceVariant);
+    if (v == kFlatVariant && !bvh.flat) v = 2;
     if ((v == 8 || v == 82 || v == 83) && !bvh.wnodes) v = 2;
     if ((v == 4 || v == 416) && !bvh.cnodes) v = 2;
     if (v >= 11 && v <= 13 && !tiny) v = 2;
@@ -387,7 +408,10 @@ void launch_trace_closest(const BvhView &bvh, const float4 *d_rays, int64_t n, f
     if (n <= 0) return;
     CRT_CHECK(n < (int64_t)1 << 31, CRT_ERR_CAPACITY, "trace batch larger than 2^31 rays");
     const int v = traversal_variant(bvh);
-    if (v >= 11 && v <= 13) {
+    if (v == kFlatVariant) {
+        k_trace_flat<ClosestJob, false><<<(int)((n + kTraceBlock - 1) / kTraceBlock), kTraceBlock, 0, s>>>(
+            ClosestJob{bvh, d_rays, d_hits}, (int)n);
+    } else if (v >= 11 && v <= 13) {
         const ClosestJob job{bvh, d_rays, d_hits};
         if (v == 13)
             launch_tiny<ClosestJob, false, 8>(job, n, false, s);
@@ -443,7 +467,10 @@ void launch_trace_shadow(const BvhView &bvh, const float *d_q, int64_t n, uint8_
     CRT_CHECK(n < (int64_t)1 << 31, CRT_ERR_CAPACITY, "trace batch larger than 2^31 queries");
     const float4 *q = reinterpret_cast<const float4 *>(d_q);
     const int v = traversal_variant(bvh);
-    if (v >= 11 && v <= 13) {
+    if (v == kFlatVariant) {
+        k_trace_flat<ShadowJob, true><<<(int)((n + kTraceBlock - 1) / kTraceBlock), kTraceBlock, 0, s>>>(
+            ShadowJob{bvh, q, d_occ, {}}, (int)n);
+    } else if (v >= 11 && v <= 13) {
         const ShadowJob job{bvh, q, d_occ, {}};
         if (v == 13)
             launch_tiny<ShadowJob, true, 8>(job, n, false, s);

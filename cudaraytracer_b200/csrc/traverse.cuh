@@ -60,7 +60,7 @@ __device__ __forceinline__ void trace_dynamic_st(Job &job, int n, Stack &st) {
     int cleft = (int)((w + 1) * n / warps) - cbase;
     // per-lane ray state
     int idx = -1;
-    BvhView bvh{nullptr, nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr, {}};
+    BvhView bvh{};
     V3 o{0.f, 0.f, 0.f}, d{0.f, 0.f, 0.f}, inv{0.f, 0.f, 0.f};
     float tmin = 0.f, t_exit = 0.f;
     Hit hit;
@@ -213,7 +213,7 @@ __device__ __forceinline__ void trace_dynamic_spec(Job &job, int n, Stack &st) {
     int cbase = (int)(w * n / warps);
     int cleft = (int)((w + 1) * n / warps) - cbase;
     int idx = -1;
-    BvhView bvh{nullptr, nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr, {}};
+    BvhView bvh{};
     V3 o{0.f, 0.f, 0.f}, d{0.f, 0.f, 0.f}, inv{0.f, 0.f, 0.f};
     float tmin = 0.f, t_exit = 0.f;
     Hit hit;
@@ -337,7 +337,7 @@ __device__ __forceinline__ void trace_dynamic8(Job &job, int n, unsigned *s_stac
     int cbase = (int)(w * n / warps);
     int cleft = (int)((w + 1) * n / warps) - cbase;
     int idx = -1;
-    BvhView bvh{nullptr, nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr, {}};
+    BvhView bvh{};
     V3 o{0.f, 0.f, 0.f}, d{0.f, 0.f, 0.f}, inv{0.f, 0.f, 0.f};
     float tmin = 0.f, t_exit = 0.f;
     unsigned oct = 0, cur = 0;
