@@ -47,6 +47,8 @@ struct BvhView {
     int *err;              // device error word (kErrTraversalBounds), or null
     const float4 *cnodes;  // the binary nodes with 16-bit quantised boxes, 2 float4 each (bvh16.cuh)
     QuantGrid grid;
+    const float4 *tri8;    // 2 float4 per triangle: v0, v1, v2.xy (32 B, one load)
+    const float2 *tri2;    // and v2.z, the original primitive index
     const float4 *flat;    // scenes of at most kFlatTris triangles: 4 float4 per triangle and the scales (flat.cuh)
 };
 
@@ -142,6 +144,21 @@ __device__ __forceinline__ void load_node(const float4 *nd, float4 &n0, float4 &
     asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(n2.x), "=f"(n2.y), "=f"(n2.z), "=f"(n2.w), "=r"(n3.x), "=r"(n3.y), "=r"(n3.z), "=r"(n3.w)
         : "l"(nd + 2));
+}
+
+// A triangle of leaf slot `slot` as one 32 B and one 8 B load: vertices in
+// a, b, c and the primitive index in a.w, as the three float4 of `tris`.
+__device__ __forceinline__ void load_tri(const BvhView &bvh, int slot, float4 &a, float4 &b, float4 &c) {
+    float x, y;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(x), "=f"(y)
+        : "l"(bvh.tri8 + 2 * (size_t)slot));
+    const float2 z = __ldg(bvh.tri2 + slot);
+    a.w = z.y;
+    b.w = c.w = 0.f;
+    c.x = x;
+    c.y = y;
+    c.z = z.x;
 }
 
 // Traversal stacks with one interface: reset / empty / push / pop of 32-bit

@@ -642,13 +642,16 @@ __global__ void __launch_bounds__(kBlock) k_small(const Task *tasks, int *idx, c
     }
 }
 
-__global__ void k_gather_tris(const float *verts, const int *idx, int n, float4 *tris) {
+__global__ void k_gather_tris(const float *verts, const int *idx, int n, float4 *tris, float4 *tri8, float2 *tri2) {
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         int p = idx[s];
         const float *v = verts + 9 * (size_t)p;
         tris[3 * (size_t)s + 0] = make_float4(v[0], v[1], v[2], __int_as_float(p));
         tris[3 * (size_t)s + 1] = make_float4(v[3], v[4], v[5], 0.f);
         tris[3 * (size_t)s + 2] = make_float4(v[6], v[7], v[8], 0.f);
+        tri8[2 * (size_t)s + 0] = make_float4(v[0], v[1], v[2], v[3]);
+        tri8[2 * (size_t)s + 1] = make_float4(v[4], v[5], v[6], v[7]);
+        tri2[s] = make_float2(v[8], __int_as_float(p));
     }
 }
 
@@ -734,6 +737,8 @@ void build_bvh(const float *d_verts, int n, cudaStream_t stream, BvhBuffers &out
     CRT_CUDA(cudaMalloc(&out.nodes, (size_t)max_nodes * 4 * sizeof(float4)));
     CRT_CUDA(cudaMalloc(&out.tris, (size_t)n * 3 * sizeof(float4)));
     CRT_CUDA(cudaMalloc(&out.slot_of_prim, (size_t)n * sizeof(int)));
+    CRT_CUDA(cudaMalloc(&out.tri8, (size_t)n * 2 * sizeof(float4)));
+    CRT_CUDA(cudaMalloc(&out.tri2, (size_t)n * sizeof(float2)));
 
     int init_keys[12];
     for (int k = 0; k < 12; ++k) init_keys[k] = (k % 6) < 3 ? INT_MAX : INT_MIN;
@@ -843,7 +848,7 @@ void build_bvh(const float *d_verts, int n, cudaStream_t stream, BvhBuffers &out
         out.num_nodes = cnt[0];
         out.depth = cnt[1];
     }
-    k_gather_tris<<<grid, kBlock, 0, stream>>>(d_verts, idx.p, n, out.tris);
+    k_gather_tris<<<grid, kBlock, 0, stream>>>(d_verts, idx.p, n, out.tris, out.tri8, out.tri2);
     k_prim_slot<<<grid, kBlock, 0, stream>>>(idx.p, n, out.slot_of_prim);
     CRT_CUDA(cudaGetLastError());
     CRT_CUDA(cudaEventRecord(e1, stream));
@@ -874,6 +879,8 @@ void free_bvh(BvhBuffers &b) {
     if (b.nodes) cudaFree(b.nodes);
     if (b.tris) cudaFree(b.tris);
     if (b.slot_of_prim) cudaFree(b.slot_of_prim);
+    if (b.tri8) cudaFree(b.tri8);
+    if (b.tri2) cudaFree(b.tri2);
     if (b.wnodes) cudaFree(b.wnodes);
     if (b.wlinks) cudaFree(b.wlinks);
     if (b.cnodes) cudaFree(b.cnodes);

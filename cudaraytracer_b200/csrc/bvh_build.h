@@ -25,9 +25,11 @@ struct BvhBuffers {
     int *err = nullptr;  // the owning context's device error word
     float4 *cnodes = nullptr;  // 16-bit quantised copy of `nodes` (bvh16.cuh)
     QuantGrid grid{};
+    float4 *tri8 = nullptr;    // the triangles again for the trace kernels (bvh.cuh, load_tri)
+    float2 *tri2 = nullptr;
     float4 *flat = nullptr;    // records of a small scene (flat.cuh), else null
     BvhView view() const {
-        return BvhView{nodes, tris, num_tris, wnodes, wlinks, (int)num_nodes, err, cnodes, grid, flat};
+        return BvhView{nodes, tris, num_tris, wnodes, wlinks, (int)num_nodes, err, cnodes, grid, tri8, tri2, flat};
     }
 };
 

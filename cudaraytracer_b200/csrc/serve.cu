@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kPathBlock, kMinBlocks) ks_paths(const SceneVi
 
 size_t scene_device_bytes(const Scene &sc) {
     const size_t n = (size_t)sc.bvh.num_tris;
-    size_t b = (size_t)sc.bvh.num_nodes * 64 + n * 48 + n * 4;  // nodes, leaf-order triangles, slot_of_prim
+    size_t b = (size_t)sc.bvh.num_nodes * 64 + n * (48 + 40) + n * 4;  // nodes, leaf-order triangles (twice), slot_of_prim
     b += (size_t)sc.bvh.num_wide_nodes * (64 + 32);            // 8-wide nodes and their child links
     b += n * 36;                                              // input vertices
     b += n * 64;                                              // shading attributes

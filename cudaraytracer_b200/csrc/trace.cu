@@ -33,7 +33,7 @@ struct ClosestJob {
         t_exit = 0.f;
     }
     __device__ void finish(int i, const BvhView &b, const Hit &h) {
-        int prim = h.slot >= 0 ? tri_prim(b, h.slot) : -1;
+        int prim = h.slot >= 0 ? __float_as_int(__ldg(b.tri2 + h.slot).y) : -1;
         hits[i] = make_float4(h.t, __int_as_float(prim), h.b1, h.b2);
     }
 };
@@ -53,7 +53,9 @@ struct ShadowJob {
         tmax = 1e8f;
         t_exit = r.t_exit;
     }
-    __device__ void finish(int i, const BvhView &b, const Hit &h) { occ[i] = shadow_ray_visible(r, b, h) ? 0 : 1; }
+    __device__ void finish(int i, const BvhView &b, const Hit &h) {
+        occ[i] = shadow_ray_visible<true>(r, b, h) ? 0 : 1;
+    }
 };
 
 // Light::Visible in two passes, with the same answer. Pass 1 looks for the
@@ -110,6 +112,25 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow(BvhView bvh, const
                                                               uint8_t *__restrict__ occ) {
     ShadowJob job{bvh, q, occ, {}};
     trace_dynamic<true>(job, n);
+}
+
+// The warp-voting traversal (trace_vote) for large batches. Bound by the L1
+// data pipe (a lane's 32 B loads are a wavefront each: about 50 nodes of two
+// and 12 triangles of two a shadow ray, 71% busy) and the latency behind it.
+// 1.31M-triangle field, 8M random rays / shadow queries, us: the lane-refill
+// kernels below 1329 / 4876; voting 1004 / 4449 (7-9 to 13.5 lanes an
+// instruction); triangles in 32 + 8 B instead of three 16 B loads and 56
+// registers for 9 x 128 threads 990 / 4221; block queues of 576 threads 946 /
+// 3944. Ordering the batch by a Morton key of the origins, leaving out the
+// sort, would give another 4-6%.
+constexpr int kVoteBlock = 576;  // 18 warps share a queue, two blocks per SM
+template <class Job>
+__global__ void __launch_bounds__(kVoteBlock, 2) k_trace_vote(Job job, int n) {
+    __shared__ int next;
+    if (threadIdx.x == 0) next = 0;
+    __syncthreads();
+    LocalStack st;
+    trace_vote<true>(job, n, st, &next);
 }
 
 // The binary traversal with its local stack, compiled for kMinBlocks
@@ -355,8 +376,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
 
 // Traversal variant of the trace kernels. The default is kFlatVariant for
 // scenes of at most kFlatTris triangles, kTinyVariant for others of at most
-// kTinyDefaultBytes and kTraceVariant otherwise;
-// CRT_TRAVERSAL overrides it.
+// kTinyDefaultBytes; otherwise kVoteVariant for batches from kVoteMinRays up
+// and kTraceVariant below; CRT_TRAVERSAL overrides it.
 //   2        binary tree, stack in local memory, per-lane refill;
 //   210/212  the same capped at 51 / 42 registers (10 / 12 blocks per SM);
 //   1        one ray per thread without refill;
@@ -375,6 +396,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
 //            per lane in shared memory.
 //   14       every triangle, no tree (k_trace_flat; scenes of at most
 //            kFlatTris triangles, else 2): the default there.
+//   15       the warp-voting traversal (k_trace_vote).
 // On the Cornell box (36 triangles, 1M random rays) 11 issues from 85% of
 // the scheduler slots with 11-12 of 32 lanes active: divergence between the
 // lanes' paths, not memory, bounds it. Capping it at 40 / 32 registers (12 /
@@ -383,12 +405,22 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_shadow8r(BvhView bvh, con
 constexpr int kTraceVariant = 2;
 constexpr int kTinyVariant = 11;
 constexpr int kFlatVariant = 14;
+constexpr int kVoteVariant = 15;
+// Smaller batches leave lanes without a second ray, and a vote only delays
+// the lanes it passes over: at 20,001 rays on a 5,120-triangle field the
+// lane-refill kernels take 22 / 49 us, voting 25 / 57; even at 200,000 (57 /
+// 132 against 59 / 131), ahead at a million (137 / 557 against 113 / 441).
+constexpr int64_t kVoteMinRays = 160 << 10;
 
-static int traversal_variant(const BvhView &bvh) {
+static int traversal_variant(const BvhView &bvh, int64_t n) {
     const char *e = getenv("CRT_TRAVERSAL");
     const int64_t tb = tiny_bytes(bvh);
     const bool tiny = tb <= kTinyBytes;
-    int v = e ? atoi(e) : bvh.flat ? kFlatVariant : (tb <= kTinyDefaultBytes ? kTinyVariant : kTraceVariant);
+    int v = e                         ? atoi(e)
+            : bvh.flat                ? kFlatVariant
+            : tb <= kTinyDefaultBytes ? kTinyVariant
+            : n >= kVoteMinRays       ? kVoteVariant
+                                      : kTraceVariant;
     if (v == kFlatVariant && !bvh.flat) v = 2;
     if ((v == 8 || v == 82 || v == 83) && !bvh.wnodes) v = 2;
     if ((v == 4 || v == 416) && !bvh.cnodes) v = 2;
@@ -404,10 +436,16 @@ static int trace_grid(const void *kernel, int64_t n) {
     return (int)(want < full ? (want > 0 ? want : 1) : full);
 }
 
+template <class Job>
+static void launch_vote(const Job &job, int64_t n, cudaStream_t s) {
+    const int full = persistent_grid((const void *)k_trace_vote<Job>, kVoteBlock);
+    k_trace_vote<<<(int)std::min<int64_t>((n + kVoteBlock - 1) / kVoteBlock, full), kVoteBlock, 0, s>>>(job, (int)n);
+}
+
 void launch_trace_closest(const BvhView &bvh, const float4 *d_rays, int64_t n, float4 *d_hits, cudaStream_t s) {
     if (n <= 0) return;
     CRT_CHECK(n < (int64_t)1 << 31, CRT_ERR_CAPACITY, "trace batch larger than 2^31 rays");
-    const int v = traversal_variant(bvh);
+    const int v = traversal_variant(bvh, n);
     if (v == kFlatVariant) {
         k_trace_flat<ClosestJob, false><<<(int)((n + kTraceBlock - 1) / kTraceBlock), kTraceBlock, 0, s>>>(
             ClosestJob{bvh, d_rays, d_hits}, (int)n);
@@ -423,6 +461,8 @@ void launch_trace_closest(const BvhView &bvh, const float4 *d_rays, int64_t n, f
     else if (v == 416)
         k_trace_closest_s<16, true><<<trace_grid((const void *)k_trace_closest_s<16, true>, n), kTraceBlock, 0, s>>>(
             bvh, d_rays, (int)n, d_hits);
+    else if (v == kVoteVariant)
+        launch_vote(ClosestJob{bvh, d_rays, d_hits}, n, s);
     else if (v == 3)
         k_trace_closest_p<<<trace_grid((const void *)k_trace_closest_p, n), kTraceBlock, 0, s>>>(bvh, d_rays, (int)n,
                                                                                                 d_hits);
@@ -466,7 +506,7 @@ void launch_trace_shadow(const BvhView &bvh, const float *d_q, int64_t n, uint8_
     if (n <= 0) return;
     CRT_CHECK(n < (int64_t)1 << 31, CRT_ERR_CAPACITY, "trace batch larger than 2^31 queries");
     const float4 *q = reinterpret_cast<const float4 *>(d_q);
-    const int v = traversal_variant(bvh);
+    const int v = traversal_variant(bvh, n);
     if (v == kFlatVariant) {
         k_trace_flat<ShadowJob, true><<<(int)((n + kTraceBlock - 1) / kTraceBlock), kTraceBlock, 0, s>>>(
             ShadowJob{bvh, q, d_occ, {}}, (int)n);
@@ -481,6 +521,8 @@ void launch_trace_shadow(const BvhView &bvh, const float *d_q, int64_t n, uint8_
     else if (v == 416)
         k_trace_shadow_s<16, true><<<trace_grid((const void *)k_trace_shadow_s<16, true>, n), kTraceBlock, 0, s>>>(
             bvh, q, (int)n, d_occ);
+    else if (v == kVoteVariant)
+        launch_vote(ShadowJob{bvh, q, d_occ, {}}, n, s);
     else if (v == 3)
         k_trace_shadow_p<<<trace_grid((const void *)k_trace_shadow_p, n), kTraceBlock, 0, s>>>(bvh, q, (int)n, d_occ);
     else if (v == 1)

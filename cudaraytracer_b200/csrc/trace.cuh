@@ -11,9 +11,19 @@ namespace crt {
 // Hit point of a closest-hit record: b0*v0 + b1*v1 + b2*v2 with
 // b0 = 1 - b1 - b2, evaluated in the reference's order
 // (Src/Core/triangle.cu:121-127).
+// kPacked reads the triangle's packed copy (load_tri), for kernels that
+// traversed it.
+template <bool kPacked = false>
 __device__ __forceinline__ V3 hit_point(const BvhView &bvh, const Hit &h) {
     const float4 *tp = bvh.tris + 3 * (size_t)h.slot;
-    float4 a = __ldg(tp + 0), b = __ldg(tp + 1), c = __ldg(tp + 2);
+    float4 a, b, c;
+    if (kPacked) {
+        load_tri(bvh, h.slot, a, b, c);
+    } else {
+        a = __ldg(tp + 0);
+        b = __ldg(tp + 1);
+        c = __ldg(tp + 2);
+    }
     float b0 = rsub(rsub(1.f, h.b1), h.b2);
     return V3{radd(radd(rmul(b0, a.x), rmul(h.b1, b.x)), rmul(h.b2, c.x)),
               radd(radd(rmul(b0, a.y), rmul(h.b1, b.y)), rmul(h.b2, c.y)),
@@ -46,10 +56,11 @@ __device__ __forceinline__ void shadow_ray_init(ShadowRay &r, V3 hp, V3 hn, V3 l
 
 // The predicate from the closest hit of closest_hit<true>(bvh, r.o, r.dir,
 // 1e-6, 1e8, r.t_exit).
+template <bool kPacked = false>
 __device__ __forceinline__ bool shadow_ray_visible(const ShadowRay &r, const BvhView &bvh, const Hit &hit) {
     if (hit.slot < 0) return true;
     if (hit.t < r.t_exit) return false;
-    V3 thp = hit_point(bvh, hit);
+    V3 thp = hit_point<kPacked>(bvh, hit);
     float td = vnorm(vsub(thp, r.l));
     if (vnorm(vsub(r.h, thp)) >= 0.1f && fabsf(rsub(td, r.sd)) >= 0.1f) return false;
     return true;

@@ -195,6 +195,126 @@ __device__ __forceinline__ void trace_dynamic_st(Job &job, int n, Stack &st) {
     }
 }
 
+// trace_dynamic with the warp voting on what to do next, over the packed
+// triangles (load_tri, bvh.cuh): a turn runs either up to kNodes node steps of the lanes that stand at an interior node or up to
+// kTris triangle tests of those that stand in a leaf, whichever the larger
+// group wants; lanes whose ray ended wait until kRefill of them are idle (or
+// nothing else is left to do) and then write their results and take new rays
+// together. Every lane's own sequence of steps is closest_hit's.
+// The block's rays are chunks of kChunk consecutive ones, gridDim chunks
+// apart (neighbouring rays stay together, expensive regions of an ordered
+// batch spread over the blocks), handed to its warps from a queue in shared
+// memory (`next`, 0 at the start): a warp with short rays takes more.
+// (4 node steps or 2 tests a turn and 8 idle lanes were the fastest of 1-8,
+// 1-4 and 4-24.)
+template <bool kCull, int kNodes = 4, int kTris = 2, int kRefill = 8, int kChunk = 64, class Job, class Stack>
+__device__ __forceinline__ void trace_vote(Job &job, int n, Stack &st, int *next) {
+    const unsigned full = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    bool left = true;
+    int idx = -1;
+    BvhView bvh{};
+    V3 o{0.f, 0.f, 0.f}, d{0.f, 0.f, 0.f}, inv{0.f, 0.f, 0.f};
+    float tmin = 0.f, t_exit = 0.f;
+    Hit hit;
+    hit.t = 0.f;
+    hit.slot = -1;
+    hit.b1 = hit.b2 = 0.f;
+    int link = kSentinel;  // node >= 0, rest of a leaf < 0, or none
+    unsigned lm[Stack::kLocal];
+    st.reset();
+    while (true) {
+        const unsigned done = __ballot_sync(full, link == kSentinel);
+        if (__popc(done) >= kRefill || done == full) {
+            if (link == kSentinel && idx >= 0) job.finish(idx, bvh, hit);
+            __syncwarp();
+            if (!left && done == full) break;
+            if (link == kSentinel) idx = -1;
+            if (left) {
+                int base = 0;
+                if (lane == 0) base = atomicAdd(next, __popc(done));
+                base = __shfl_sync(full, base, 0);
+                const int v = base + __popc(done & lt);
+                const int64_t i = ((int64_t)(v / kChunk) * gridDim.x + blockIdx.x) * kChunk + v % kChunk;
+                if (link == kSentinel && i < n) {
+                    idx = (int)i;
+                    float tmax;
+                    job.setup(idx, bvh, o, d, tmin, tmax, t_exit);
+                    inv = v3(rrcp(d.x), rrcp(d.y), rrcp(d.z));
+                    hit.t = tmax;
+                    hit.slot = -1;
+                    hit.b1 = hit.b2 = 0.f;
+                    st.reset();
+                    link = 0;
+                }
+                left = __all_sync(full, link != kSentinel);  // a lane without a ray: none are left
+            }
+            __syncwarp();
+        }
+        const unsigned at_node = __ballot_sync(full, link >= 0);
+        const unsigned at_leaf = __ballot_sync(full, link < 0 && link != kSentinel);
+        if (__popc(at_node) >= __popc(at_leaf)) {
+#pragma unroll 1
+            for (int rep = 0; rep < kNodes; ++rep) {
+                if (link < 0) break;
+                if (link >= bvh.num_nodes || st.sp >= kStackSize) {
+                    report_traversal_bounds(bvh);
+                    link = kSentinel;
+                    break;
+                }
+                float4 n0, n1, n2;
+                int4 n3;
+                load_node(bvh.nodes + 4 * (size_t)link, n0, n1, n2, n3);
+                float t0, t1;
+                const bool h0 = slab(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, o, inv, tmin, hit.t, t0);
+                const bool h1 = slab(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, o, inv, tmin, hit.t, t1);
+                if (h0 && h1) {
+                    int near = n3.x, far = n3.y;
+                    if (t1 < t0) {
+                        near = n3.y;
+                        far = n3.x;
+                    }
+                    st.push((unsigned)far, lm);
+                    link = near;
+                } else if (h0) {
+                    link = n3.x;
+                } else if (h1) {
+                    link = n3.y;
+                } else {
+                    link = st.empty() ? kSentinel : (int)st.pop(lm);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int rep = 0; rep < kTris; ++rep) {
+                if (link >= 0 || link == kSentinel) break;
+                const int code = ~link;
+                const int slot = code >> 4, count = code & 15;
+                bool next = count == 0;
+                if (!next) {
+                    if (slot + count > bvh.num_tris) {
+                        report_traversal_bounds(bvh);
+                        link = kSentinel;
+                        break;
+                    }
+                    float4 a, b, c;
+                    load_tri(bvh, slot, a, b, c);
+                    const bool acc = intersect_triangle<kCull>(o, d, a, b, c, slot, hit);
+                    if (acc && hit.t < t_exit) {
+                        link = kSentinel;
+                        break;
+                    }
+                    link = leaf_link(slot + 1, count - 1);
+                    next = count == 1;
+                }
+                if (next) link = st.empty() ? kSentinel : (int)st.pop(lm);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // trace_dynamic with postponed leaves (the speculative while-while loop of
 // Aila and Laine, "Understanding the Efficiency of Ray Traversal on GPUs",
 // HPG 2009): a lane that reaches a leaf keeps it pending and goes on
