@@ -50,31 +50,6 @@ static __device__ __noinline__ void flat_tree(const BvhView &bvh, V3 o, V3 d, fl
     hit = closest_hit<kEarlyExit>(bvh, o, d, tmin, tmax, t_exit);
 }
 
-// Two products and sums per instruction.
-struct F2 {
-    unsigned long long v;
-};
-__device__ __forceinline__ F2 f2(float a, float b) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ F2 f2fma(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
-}
-__device__ __forceinline__ F2 f2mul(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ float2 f2get(F2 a) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
-    return r;
-}
-
 // Copies a scene's records into the block's shared memory (the caller
 // synchronises the block afterwards).
 constexpr int kFlatWords = 8 * (kFlatTris / 2) + 1;

@@ -247,10 +247,13 @@ struct TemporalArgs {
     bool first;
 };
 
+// 64 registers (4 blocks of 256 per SM) instead of 80: the taps' dependent
+// loads bound it, and a third more warps bring it from 198 to 169 us at
+// 1920 x 1080.
 // TemporalDenoising (renderer.cuh:524-677). Reads the noisy frame, writes
 // the blended result both as the frame's working buffer and as the next
 // frame's history, and the pixel's edge-stopping record.
-__global__ void k_svgf_temporal(TemporalArgs a, GB cur, GB last, EdgeOut eo) {
+__global__ void __launch_bounds__(256, 4) k_svgf_temporal(TemporalArgs a, GB cur, GB last, EdgeOut eo) {
     int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= a.W || y >= a.H) return;
     int idx = y * a.W + x;
@@ -388,6 +391,7 @@ struct VarianceArgs {
     const float2 *mom_d, *mom_i;
     const float4 *edge;
     const int2 *tag;
+    float2 *var;  // the two variances again, for the a-trous passes' pre-blur
 };
 
 // Tap sources for the variance body (global memory or a shared tile).
@@ -491,6 +495,14 @@ __device__ __forceinline__ void variance_pixel(const VarianceArgs &a, const GB &
     vi *= 4.f / h;
     a.out_d[idx] = make_float4(fd.x, fd.y, fd.z, vd);
     a.out_i[idx] = make_float4(fi.x, fi.y, fi.z, vi);
+    a.var[idx] = make_float2(vd, vi);
+}
+
+// A pixel with enough history passes through.
+__device__ __forceinline__ void variance_copy(const VarianceArgs &a, int idx, float4 d, float4 i) {
+    a.out_d[idx] = d;
+    a.out_i[idx] = i;
+    a.var[idx] = make_float2(d.w, i.w);
 }
 
 // One thread per pixel, taps from global memory.
@@ -500,8 +512,7 @@ __global__ void k_svgf_variance(VarianceArgs a, GB g) {
     int idx = y * a.W + x;
     const int2 ctag = a.tag[idx];
     if (ctag.y >= 4) {
-        a.out_d[idx] = a.in_d[idx];
-        a.out_i[idx] = a.in_i[idx];
+        variance_copy(a, idx, a.in_d[idx], a.in_i[idx]);
         return;
     }
     variance_pixel(a, g, VarGlobalTaps{a}, x, y, ctag.y, ctag.x);
@@ -524,10 +535,7 @@ __global__ void __launch_bounds__(kVarTileX * kVarTileY) k_svgf_variance_tiled(V
     if (inside) ctag = a.tag[y * a.W + x];
     const bool filter = inside && ctag.y < 4;
     if (!__syncthreads_or(filter)) {
-        if (inside) {
-            a.out_d[y * a.W + x] = a.in_d[y * a.W + x];
-            a.out_i[y * a.W + x] = a.in_i[y * a.W + x];
-        }
+        if (inside) variance_copy(a, y * a.W + x, a.in_d[y * a.W + x], a.in_i[y * a.W + x]);
         return;
     }
     const int tid = threadIdx.y * kVarTileX + threadIdx.x;
@@ -546,8 +554,7 @@ __global__ void __launch_bounds__(kVarTileX * kVarTileY) k_svgf_variance_tiled(V
     if (!inside) return;
     if (!filter) {
         const VarTileTaps t{sd, si, se, sm, stg, bx - R, by - R, RW};
-        a.out_d[y * a.W + x] = t.d(x, y);
-        a.out_i[y * a.W + x] = t.i(x, y);
+        variance_copy(a, y * a.W + x, t.d(x, y), t.i(x, y));
         return;
     }
     variance_pixel(a, g, VarTileTaps{sd, si, se, sm, stg, bx - R, by - R, RW}, x, y, ctag.y, ctag.x);
@@ -562,25 +569,13 @@ struct AtrousArgs {
     const int2 *tag;
 };
 
-// Tap sources for the a-trous body: straight from global memory, or from a
-// shared-memory tile that covers the block and its halo.
+// Tap source of the a-trous body below.
 struct GlobalTaps {
     const AtrousArgs &a;
     __device__ __forceinline__ float4 d(int x, int y) const { return a.in_d[y * a.W + x]; }
     __device__ __forceinline__ float4 i(int x, int y) const { return a.in_i[y * a.W + x]; }
     __device__ __forceinline__ float4 e(int x, int y) const { return a.edge[y * a.W + x]; }
     __device__ __forceinline__ int2 t(int x, int y) const { return a.tag[y * a.W + x]; }
-};
-
-struct TileTaps {
-    const float4 *sd, *si, *se;
-    const int2 *st;
-    int x0, y0, rw;  // tile origin (image coordinates of its first element) and row width
-    __device__ __forceinline__ int at(int x, int y) const { return (y - y0) * rw + (x - x0); }
-    __device__ __forceinline__ float4 d(int x, int y) const { return sd[at(x, y)]; }
-    __device__ __forceinline__ float4 i(int x, int y) const { return si[at(x, y)]; }
-    __device__ __forceinline__ float4 e(int x, int y) const { return se[at(x, y)]; }
-    __device__ __forceinline__ int2 t(int x, int y) const { return st[at(x, y)]; }
 };
 
 // AtrousKernel (renderer.cuh:807-954) for pixel (x, y): 3x3 pre-blur of
@@ -673,40 +668,159 @@ __device__ __forceinline__ void atrous_pixel(const AtrousArgs &a, const GB &g, c
         a.out_i[idx] = make_float4(ci.x, ci.y, ci.z, 1.f);
 }
 
-// One thread per pixel, taps from global memory (large steps).
+// One thread per pixel, taps from global memory (CRT_SVGF_TILED=0).
 __global__ void k_svgf_atrous(AtrousArgs a, GB g) {
     int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= a.W || y >= a.H) return;
     atrous_pixel(a, g, GlobalTaps{a}, x, y);
 }
 
-// Small steps (1 and 2): the block's kTileX x kTileY pixels and their halo
-// of 2 * kStep (the 5x5 taps; it also covers the 3x3 pre-blur) are staged
-// once in shared memory (colour, variance, edge record and tag: 56 B per
-// pixel), so each loaded pixel serves up to 25 taps of the block instead
-// of being fetched per tap.
 constexpr int kTileX = 32, kTileY = 8;
 
-template <int kStep>
-__global__ void __launch_bounds__(kTileX * kTileY) k_svgf_atrous_tiled(AtrousArgs a, GB g) {
-    constexpr int R = 2 * kStep, RW = kTileX + 2 * R, RH = kTileY + 2 * R, N = RW * RH;
-    __shared__ float4 sd[N], si[N], se[N];
-    __shared__ int2 stg[N];
-    const int bx = blockIdx.x * kTileX, by = blockIdx.y * kTileY;
+// Every step from a shared-memory tile: at step s the taps of a pixel lie on
+// its own sub-lattice of pixels s apart, so a block takes 32 x 8 pixels of
+// one sub-lattice (kPair, s > 1: of two that neighbour in x, so that loads
+// fill their 32 B sectors) and a halo of two lattice points, whatever the
+// step. Per pixel: direct and indirect colours interleaved (the two halves of
+// each packed instruction), normal and depth, ids, history length. Pixels
+// outside the image have a zero normal, which gives them weight 0. The 3x3
+// pre-blur of the variance, which is at unit distance, reads the variance
+// planes that the pass before wrote beside its colours.
+//
+// Bound by issue (25 taps). 1920 x 1080, us per pass at steps 1, 2, 4, 8, 16:
+// 168, 170, 173, 184, 203; as scalar code with bounds checks per tap, over
+// tiles of float4 planes (steps 1, 2) or global memory (4, 8, 16), it was
+// 228, 233, 266, 271, 256.
+struct VarPlanes {
+    const float2 *in;
+    float2 *out;
+};
+
+__device__ __forceinline__ float lg2_approx(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+template <bool kPair>
+__global__ void __launch_bounds__(kTileX * kTileY) k_svgf_atrous_lattice(AtrousArgs a, GB g, VarPlanes vp) {
+    constexpr int kLanes = kPair ? 2 : 1;                 // sub-lattices in x
+    constexpr int RW = kTileX + 4 * kLanes, RH = kTileY + 4, N = RW * RH;
+    __shared__ float4 s_rg[N], s_bv[N], s_e[N];  // (d.r, i.r, d.g, i.g), (d.b, i.b, d.var, i.var), (normal, depth)
+    __shared__ int s_id[N], s_h[N];
+    const int step = a.step, px = step / kLanes;          // kPair: pairs of sub-lattices per period
+    // the block's first pixel: its tile of 32 / kLanes x 8 lattice points
+    // and the sub-lattice within the period
+    const int bx = ((int)blockIdx.x / px) * (kTileX / kLanes) * step + ((int)blockIdx.x % px) * kLanes;
+    const int by = ((int)blockIdx.y / step) * kTileY * step + (int)blockIdx.y % step;
     const int tid = threadIdx.y * kTileX + threadIdx.x;
     for (int k = tid; k < N; k += kTileX * kTileY) {
-        const int gx = bx - R + k % RW, gy = by - R + k / RW;
-        if (gx < 0 || gx >= a.W || gy < 0 || gy >= a.H) continue;  // never read: taps check the image bounds
-        const int gi = gy * a.W + gx;
-        sd[k] = a.in_d[gi];
-        si[k] = a.in_i[gi];
-        se[k] = a.edge[gi];
-        stg[k] = a.tag[gi];
+        const int cx = k % RW, cy = k / RW;
+        const int gx = bx + (cx / kLanes - 2) * step + cx % kLanes, gy = by + (cy - 2) * step;
+        float4 rg = make_float4(0.f, 0.f, 0.f, 0.f), bv = rg, e = rg;
+        int2 t = make_int2(0, 1);
+        if (gx >= 0 && gx < a.W && gy >= 0 && gy < a.H) {
+            const int gi = gy * a.W + gx;
+            const float4 d = a.in_d[gi], i = a.in_i[gi];
+            rg = make_float4(d.x, i.x, d.y, i.y);
+            bv = make_float4(d.z, i.z, d.w, i.w);
+            e = a.edge[gi];
+            t = a.tag[gi];
+        }
+        s_rg[k] = rg;
+        s_bv[k] = bv;
+        s_e[k] = e;
+        s_id[k] = t.x;
+        s_h[k] = t.y;
+    }
+    const int x = bx + ((int)threadIdx.x / kLanes) * step + (int)threadIdx.x % kLanes, y = by + (int)threadIdx.y * step;
+    const bool inside = x < a.W && y < a.H;
+    const int idx = y * a.W + x;
+    // 3x3 blur of the variance at unit distance
+    float fvd = 0.f, fvi = 0.f, fvw = 0.f, dz = 0.f;
+    if (inside) {
+        dz = fmaxf(g.motion_depth[idx].w, 1e-4f);
+#pragma unroll
+        for (int vj = -1; vj <= 1; vj++)
+#pragma unroll
+            for (int vi = -1; vi <= 1; vi++) {
+                const int sx = x + vi, sy = y + vj;
+                if (sx < 0 || sx >= a.W || sy < 0 || sy >= a.H) continue;
+                const float w = (vi ? 0.25f : 0.5f) * (vj ? 0.25f : 0.5f);
+                const float2 v = vp.in[sy * a.W + sx];
+                fvd += w * fmaxf(0.f, v.x);
+                fvi += w * fmaxf(0.f, v.y);
+                fvw += w;
+            }
     }
     __syncthreads();
-    const int x = bx + threadIdx.x, y = by + threadIdx.y;
-    if (x >= a.W || y >= a.H) return;
-    atrous_pixel(a, g, TileTaps{sd, si, se, stg, bx - R, by - R, RW}, x, y);
+    if (!inside) return;
+    fvw = fmaxf(fvw, 1e-6f);
+    const float sdd = sqrtf(fvd / fvw) + 1e-3f, sdi = sqrtf(fvi / fvw) + 1e-3f;
+    const int c = ((int)threadIdx.y + 2) * RW + (int)threadIdx.x + 2 * kLanes;
+    const float4 crg = s_rg[c], cbv = s_bv[c], ce = s_e[c];
+    const int cid = s_id[c], ch = max(s_h[c], 1);
+    const float cdl = luminance(V3{crg.x, crg.z, cbv.x}), cil = luminance(V3{crg.y, crg.w, cbv.y});
+    const float boot = fminf(1.f, fmaxf(0.f, (4.f - (float)ch) / 3.f));
+    const float sdep = fmaxf(a.sigma_depth, 1e-3f) * fmaxf(dz, 1e-4f) * (1.f + 2.5f * boot);
+    const float sld = a.sigma_light * (1.f + 2.0f * boot), sli = a.sigma_light * (1.f + 1.5f * boot);
+    const float sn = fmaxf(8.f, a.sigma_normal * (1.f - 0.85f * boot));
+    // exponents in base 2: -|dz| / (sdep dist + 1e-6), -|dl| sqrt(ref) /
+    // (sld sdd) and the indirect term's factor, times log2 e
+    const float ld = kLog2e / (sld * sdd), li = kLog2e * sqrtf(fmaxf(cil, 1e-4f)) / (sli * sdi);
+    float iz[6];
+    {
+        const float dist[6] = {0.f, 1.f, 1.41421356f, 2.f, 2.23606798f, 2.82842712f};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) iz[k] = kLog2e / (sdep * (dist[k] * step) + 1e-6f);
+    }
+    const F2 lr = f2(0.2126f, 0.2126f), lgc = f2(0.7152f, 0.7152f), lb = f2(0.0722f, 0.0722f);
+    F2 ar = f2(0.f, 0.f), ag = ar, ab = ar, tw = ar, av = ar;
+#pragma unroll
+    for (int kj = -2; kj <= 2; kj++)
+#pragma unroll
+        for (int ki = -2; ki <= 2; ki++) {
+            const int k = c + kj * RW + ki * kLanes;
+            if (s_id[k] != cid) continue;
+            const ulonglong2 rg = *reinterpret_cast<const ulonglong2 *>(&s_rg[k]);
+            const ulonglong2 bv = *reinterpret_cast<const ulonglong2 *>(&s_bv[k]);
+            const float4 e = s_e[k];
+            constexpr float kw[3] = {3.f / 8.f, 1.f / 4.f, 1.f / 16.f};
+            constexpr int zi[3][3] = {{0, 1, 3}, {1, 2, 4}, {3, 4, 5}};
+            const int ai = ki < 0 ? -ki : ki, aj = kj < 0 ? -kj : kj;
+            const float2 nl = f2get(f2fma(F2{rg.x}, lr, f2fma(F2{rg.y}, lgc, f2mul(F2{bv.x}, lb))));
+            const float n_dot = fmaxf(0.f, dot(V3{ce.x, ce.y, ce.z}, V3{e.x, e.y, e.z}));
+            const float base = fmaf(sn, lg2_approx(n_dot), -fabsf(ce.w - e.w) * iz[zi[aj][ai]]);
+            const float dref = sqrt_approx(fmaxf(fmaxf(cdl, nl.x), 1e-4f));
+            float w = kw[ai] * kw[aj];
+            if (boot > 0.f) w *= 0.5f + 0.5f * fminf((float)max(s_h[k], 1) / 4.f, 1.f);
+            const float dw = ex2_approx(fmaf(-fabsf(cdl - nl.x) * dref, ld, base)) * w;
+            const float iw = ex2_approx(fmaf(-fabsf(cil - nl.y), li, base)) * w;
+            const F2 w2 = f2(dw, iw);
+            const float2 v = f2get(F2{bv.y});
+            ar = f2fma(w2, F2{rg.x}, ar);
+            ag = f2fma(w2, F2{rg.y}, ag);
+            ab = f2fma(w2, F2{bv.x}, ab);
+            tw = f2add(tw, w2);
+            av = f2fma(f2mul(w2, w2), f2(fmaxf(0.f, v.x), fmaxf(0.f, v.y)), av);
+        }
+    const float2 r = f2get(ar), gg = f2get(ag), b = f2get(ab), t = f2get(tw), vv = f2get(av);
+    float4 od = make_float4(crg.x, crg.z, cbv.x, 1.f), oi = make_float4(crg.y, crg.w, cbv.y, 1.f);
+    if (t.x > 1e-6f) od = make_float4(r.x / t.x, gg.x / t.x, b.x / t.x, vv.x / (t.x * t.x));
+    if (t.y > 1e-6f) oi = make_float4(r.y / t.y, gg.y / t.y, b.y / t.y, vv.y / (t.y * t.y));
+    a.out_d[idx] = od;
+    a.out_i[idx] = oi;
+    if (vp.out) vp.out[idx] = make_float2(od.w, oi.w);
 }
 
 // ---------------------------------------------------------------------------
@@ -728,6 +842,7 @@ void SvgfState::allocate(int w, int h) {
     }
     CRT_CUDA(cudaMalloc(&edge, n * sizeof(float4)));
     CRT_CUDA(cudaMalloc(&tag, n * sizeof(int2)));
+    for (int k = 0; k < 2; ++k) CRT_CUDA(cudaMalloc(&var[k], n * sizeof(float2)));
     reset_sync();
 }
 
@@ -747,6 +862,8 @@ void SvgfState::reset_sync() {
 void SvgfState::release() {
     if (edge) cudaFree(edge), edge = nullptr;
     if (tag) cudaFree(tag), tag = nullptr;
+    for (int k = 0; k < 2; ++k)
+        if (var[k]) cudaFree(var[k]), var[k] = nullptr;
     for (int k = 0; k < 2; ++k) {
         for (void **p : {(void **)&buf_d[k], (void **)&buf_i[k], (void **)&hist_d[k], (void **)&hist_i[k],
                          (void **)&mom_d[k], (void **)&mom_i[k], (void **)&hlen[k]})
@@ -761,7 +878,7 @@ int svgf_frame(SvgfState &st, const DenoiseParams &p, const GBufferPlanes &cur, 
                const float4 *noisy_d, const float4 *noisy_i, float4 *out_d, float4 *out_i, cudaStream_t s) {
     const int W = st.W, H = st.H;
     dim3 b(16, 16), g((W + 15) / 16, (H + 15) / 16);
-    dim3 bt(kTileX, kTileY), gt((W + kTileX - 1) / kTileX, (H + kTileY - 1) / kTileY);
+    const dim3 bt(kTileX, kTileY);
     // CRT_SVGF_TILED=0 runs every a-trous pass from global memory
     const char *tv = getenv("CRT_SVGF_TILED");
     const bool tiled = !(tv && tv[0] == '0');
@@ -809,6 +926,7 @@ int svgf_frame(SvgfState &st, const DenoiseParams &p, const GBufferPlanes &cur, 
     va.mom_i = st.mom_i[t];
     va.edge = st.edge;
     va.tag = st.tag;
+    va.var = st.var[c];
     if (tiled && va.half == kVarHalf)
         k_svgf_variance_tiled<<<dim3((W + kVarTileX - 1) / kVarTileX, (H + kVarTileY - 1) / kVarTileY),
                                 dim3(kVarTileX, kVarTileY), 0, s>>>(va, gc);
@@ -831,11 +949,15 @@ int svgf_frame(SvgfState &st, const DenoiseParams &p, const GBufferPlanes &cur, 
         aa.out_i = last_pass ? out_i : st.buf_i[1 - c];
         aa.edge = st.edge;
         aa.tag = st.tag;
-        if (aa.step == 1 && tiled)
-            k_svgf_atrous_tiled<1><<<gt, bt, 0, s>>>(aa, gc);
-        else if (aa.step == 2 && tiled)
-            k_svgf_atrous_tiled<2><<<gt, bt, 0, s>>>(aa, gc);
-        else
+        const VarPlanes vp{st.var[1 - c], last_pass ? nullptr : st.var[c]};
+        if (tiled && aa.step == 1) {
+            const dim3 gt((W + kTileX - 1) / kTileX, (H + kTileY - 1) / kTileY);
+            k_svgf_atrous_lattice<false><<<gt, bt, 0, s>>>(aa, gc, vp);
+        } else if (tiled) {
+            const int period_x = kTileX / 2 * aa.step, period_y = kTileY * aa.step;
+            const dim3 gt((W + period_x - 1) / period_x * (aa.step / 2), (H + period_y - 1) / period_y * aa.step);
+            k_svgf_atrous_lattice<true><<<gt, bt, 0, s>>>(aa, gc, vp);
+        } else
             k_svgf_atrous<<<g, b, 0, s>>>(aa, gc);
         ++launches;
         c = 1 - c;

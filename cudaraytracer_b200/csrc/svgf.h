@@ -32,6 +32,7 @@ struct SvgfState {
     int *hlen[2] = {};
     float4 *edge = nullptr;  // per-pixel decoded normal + depth of the current frame
     int2 *tag = nullptr;     // per-pixel material | mesh << 16, history length
+    float2 *var[2] = {};     // direct and indirect variance, ping-pong as the buffers
     int t = 0;
     bool first = true;
     void allocate(int w, int h);
