@@ -50,7 +50,7 @@ struct ConvArgs {
     int Ng, groups;             // output channels of one CTA and N / Ng
     int Ws, R, P, TS;           // block: strip width, rows, row pitch Ws + 2, positions between tile starts
     int KCs, nst, S;            // channels per stage, stages per block (C / KCs), stage buffers
-    int flip, relu, resident;
+    int flip, relu, resident, by_tile;
     int vec32, vec_f32;         // out and mask 32-byte aligned; out_f32 16-byte aligned
     uint32_t region_bytes;      // one layout chunk of a stage: (R + 2) P rows, rounded up to 1 KB
     uint32_t stage_bytes, wres_bytes;
@@ -214,7 +214,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         fill(k);
     };
     volatile int *abort = &abort_flag;
-    const bool by_tile = a.nst > 1;  // how the two MMA warps share the work
+    // How the two MMA warps share the work: alternate tiles, or alternate
+    // blocks. A barrier's phases are told apart by parity only, so whoever
+    // waits on one must see every phase of it: each accumulator belongs to one
+    // MMA warp (by tiles: the warp of its parity; by blocks: half of them each)
+    // and to one epilogue group (of its parity), and by blocks, S being even,
+    // so does each stage buffer.
+    const bool by_tile = a.by_tile;
+    const uint32_t half_slots = a.slots >> 1;
 
     if (tid == 0) {
         for (int i = 0; i < S; ++i) {
@@ -314,9 +321,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         };
         int buf = 0;  // stage buffer and the parity of its next phase
         uint32_t buf_par = 0;
-        // the block's first tile, its accumulator and the parity of that
-        // accumulator's release (a fresh barrier passes a wait for parity 1)
-        uint32_t slot0 = 0, par0 = 1;
+        // this warp's accumulators [lo, hi), the next of them and the parity
+        // of its release (a fresh barrier passes a wait for parity 1)
+        const uint32_t lo = by_tile ? 0 : group * half_slots, hi = by_tile ? a.slots : lo + half_slots;
+        uint32_t slot0 = lo, par0 = 1;
         const uint32_t tstep = by_tile ? 2 : 1;
         bool run = !a.resident || wait(&wbar, 0);
         Block k = first_block();
@@ -336,8 +344,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     bdesc0 + (a.resident ? (uint32_t)(st * (a.KCs >> kcl)) * wch16 : buf * stage16);
                 uint32_t slot = slot0 + first, par = par0;
                 for (uint32_t t = first; t < tiles; t += tstep, ad += tstep * ts16, slot += tstep) {
-                    if (slot >= a.slots) {
-                        slot -= a.slots;
+                    if (slot >= hi) {
+                        slot -= hi - lo;
                         par ^= 1;
                     }
                     if (st == 0) {
@@ -390,7 +398,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 buf = 0;
                 buf_par ^= 1;
             }
-            for (slot0 += tiles; slot0 >= a.slots; slot0 -= a.slots) par0 ^= 1;
+            if (mine)
+                for (slot0 += tiles; slot0 >= hi; slot0 -= hi - lo) par0 ^= 1;
         }
         // every MMA issued has finished before TMEM is released
         tc::mma_commit_pred(leader, tc::smem_addr(&mma_done[group]));
@@ -399,16 +408,22 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         // ---- epilogue: one thread per pixel of the tile ----
         const int q = warp & 3;
         const uint32_t group = (uint32_t)(warp - 3) >> 2;
-        uint32_t slot = group, par = 0, mine = group;  // mine = 0: the next tile is this group's
+        // next accumulator and its parity, of all blocks or (by blocks) of the
+        // even and of the odd ones
+        uint32_t next_slot[2] = {0, half_slots}, next_par[2] = {0, 0};
         bool run = true;
         Block k = first_block();
         for (int b = b_beg; b < b_end && run; ++b, next_block(k)) {
+            const bool odd = !by_tile && ((b - b_beg) & 1);
+            const uint32_t lo = odd ? half_slots : 0, hi = by_tile || odd ? a.slots : half_slots;
+            uint32_t at = odd ? next_slot[1] : next_slot[0], at_par = odd ? next_par[1] : next_par[0];
             for (int t = 0; t < k.tiles; ++t) {
-                if (mine) {
-                    mine = 0;
-                    continue;
+                const uint32_t slot = at, par = at_par;
+                if (++at == hi) {
+                    at = lo;
+                    at_par ^= 1;
                 }
-                mine = 1;
+                if ((slot & 1) != group) continue;
                 if (!tc::mbar_wait_or_abort(&tfull[slot], par, abort)) {
                     run = false;
                     break;
@@ -439,12 +454,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&tempty[slot]);  // this quarter's TMEM reads are done
-                slot += 2;  // an even number of accumulators
-                if (slot >= a.slots) {
-                    slot -= a.slots;
-                    par ^= 1;
-                }
             }
+            next_slot[0] = odd ? next_slot[0] : at;
+            next_par[0] = odd ? next_par[0] : at_par;
+            next_slot[1] = odd ? at : next_slot[1];
+            next_par[1] = odd ? at_par : next_par[1];
         }
     }
     tc::fence_before_sync();
@@ -994,7 +1008,9 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
     a.TS = pl.TS;
     a.KCs = pl.KCs;
     a.nst = C / pl.KCs;
-    a.S = pl.S;
+    // (by blocks each warp needs two buffers of its own to load ahead)
+    a.by_tile = a.nst > 1 || pl.S < 4;
+    a.S = a.by_tile ? pl.S : 4;
     a.flip = flip ? 1 : 0;
     a.relu = relu ? 1 : 0;
     a.resident = pl.resident;
