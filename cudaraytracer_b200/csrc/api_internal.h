@@ -57,9 +57,20 @@ struct crt_ctx {
 
 namespace crt {
 // Tensor-core 3x3 convolutions (conv.cu).
+// What a forward layer's epilogue does beside storing its output: the same
+// pixels again (or, with up2, each at its four places of an image of twice
+// the size) at out2 with out2_pitch channels per pixel, or the 5x5 filter of
+// its 32 channels as logits over noisy into filtered (then no out_f32).
+struct ConvExtra {
+    __nv_bfloat16 *out2 = nullptr;
+    int out2_pitch = 0;
+    bool up2 = false;
+    const float4 *noisy = nullptr;
+    float4 *filtered = nullptr;
+};
 void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const float *bias, const __nv_bfloat16 *mask,
                     __nv_bfloat16 *out, float *out_f32, int *err, int nimg, int h, int w, int C, int N, bool flip,
-                    bool relu, cudaStream_t s);
+                    bool relu, cudaStream_t s, const ConvExtra &x = {});
 void conv3x3_wgrad_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *g, float *dw, int *err, int nimg, int h, int w,
                           int C, int N, cudaStream_t s);
 }  // namespace crt

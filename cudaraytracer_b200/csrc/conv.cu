@@ -23,6 +23,7 @@
 //                         MN-major operands, FP32 atomics into dW.
 #include "api_internal.h"
 #include "tc.cuh"
+#include "kpcn_filter.cuh"
 #include <algorithm>
 #include <cstring>
 #include <utility>
@@ -51,6 +52,7 @@ struct ConvArgs {
     int Ws, R, P, TS;           // block: strip width, rows, row pitch Ws + 2, positions between tile starts
     int KCs, nst, S;            // channels per stage, stages per block (C / KCs), stage buffers
     int flip, relu, resident, by_tile;
+    ConvExtra x;
     int vec32, vec_f32;         // out and mask 32-byte aligned; out_f32 16-byte aligned
     uint32_t region_bytes;      // one layout chunk of a stage: (R + 2) P rows, rounded up to 1 KB
     uint32_t stage_bytes, wres_bytes;
@@ -71,7 +73,8 @@ __device__ __forceinline__ void store32(void *p, const uint32_t (&v)[8]) {
 
 // The epilogue of 16 consecutive channels of one pixel (offset o of the
 // output): bias and ReLU in FP32, then BF16 (times the mask) and / or FP32.
-__device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, const float *bias, size_t o) {
+__device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, const float *bias, size_t o,
+                                             __nv_bfloat16 *o2) {
     float r[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -105,6 +108,15 @@ __device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, 
             const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&m[i]));
             if (!(f.x > 0.f)) w[i] &= 0xffff0000u;
             if (!(f.y > 0.f)) w[i] &= 0x0000ffffu;
+        }
+    }
+    if (o2) {  // 32-byte aligned
+        store32(o2, w);
+        if (a.x.up2) {
+            const size_t row = (size_t)2 * a.wd * a.x.out2_pitch;
+            store32(o2 + a.x.out2_pitch, w);
+            store32(o2 + row, w);
+            store32(o2 + row + a.x.out2_pitch, w);
         }
     }
     __nv_bfloat16 *dst = a.out + o;
@@ -160,7 +172,8 @@ __device__ __forceinline__ void conv_store16(const ConvArgs &a, const float *v, 
 // The order of the sums is fixed per layer shape (ConvOrder) and does not
 // depend on the tiling: kKK = K steps per channel chunk of the order, kRows:
 // tap rows outside the channel chunks, else the channel chunks outermost.
-template <int kKK, bool kRows>
+// kFilter: the epilogue applies the 5x5 filter (ConvExtra).
+template <int kKK, bool kRows, bool kFilter = false>
 __global__ void __launch_bounds__(kConvThreads, 1)
     k_conv3x3(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_w, ConvArgs a,
               int kcl) {
@@ -433,7 +446,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 const int pos = t * a.TS + q * 32 + lane;
                 const int row = pos / P, col = pos - row * P;
                 const bool valid = row < k.rows && col < k.w;
-                const size_t o = (((size_t)k.img * H + k.y0 + row) * W + k.x0 + col) * N + n0;
+                const int y = k.y0 + row, x = k.x0 + col;
+                const size_t o = (((size_t)k.img * H + y) * W + x) * N + n0;
+                __nv_bfloat16 *o2 = nullptr;
+                if (a.x.out2)
+                    o2 = a.x.out2 + n0 +
+                         (a.x.up2 ? ((size_t)k.img * 2 * H + 2 * y) * 2 * W + 2 * x : ((size_t)k.img * H + y) * W + x) *
+                             a.x.out2_pitch;
                 const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + slot * a.slot_cols;
                 for (int c = 0; c < Ng; c += 32) {
                     float v[32];
@@ -446,9 +465,17 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 #pragma unroll
                         for (int i = 0; i < 16; ++i) v[i] = h16[i];
                     }
-                    if (valid) {
-                        conv_store16(a, v, s_bias + c, o + c);
-                        if (c + 32 <= Ng) conv_store16(a, v + 16, s_bias + c + 16, o + c + 16);
+                    if (kFilter && valid) {  // one group of 32 channels, 25 of them logits
+                        float wt[kTaps5];
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] += s_bias[i];
+                        softmax25(v, wt);
+                        const size_t img = (size_t)k.img * H * W;
+                        a.x.filtered[img + (size_t)y * W + x] = filter25(wt, a.x.noisy + img, x, y, H, W);
+                    } else if (valid) {
+                        conv_store16(a, v, s_bias + c, o + c, o2 ? o2 + c : nullptr);
+                        if (c + 32 <= Ng)
+                            conv_store16(a, v + 16, s_bias + c + 16, o + c + 16, o2 ? o2 + c + 16 : nullptr);
                     }
                 }
                 tc::fence_before_sync();
@@ -880,11 +907,12 @@ struct ConvPlan {
 // (their results are dropped).
 size_t conv_over_rows(int tiles, int TS, int R, int P) { return (size_t)std::max(0, (tiles - 1) * TS + 130 - R * P); }
 
-ConvPlan conv_plan(const ConvOrder &ord, int nimg, int h, int w, int C, int N, int sms) {
+// one_group: all output channels in one CTA (the filter needs a pixel's 32).
+ConvPlan conv_plan(const ConvOrder &ord, int nimg, int h, int w, int C, int N, int sms, bool one_group) {
     ConvPlan best{};
     best.cost = 1e30;
     const size_t cap = 227 * 1024 - 1024 - 4096;  // minus base alignment and static shared memory
-    for (int groups = 1; groups <= N / 16; ++groups) {
+    for (int groups = 1; groups <= (one_group ? 1 : N / 16); ++groups) {
         if (N % (16 * groups)) continue;
         const int Ng = N / groups;
         const size_t wall = (size_t)18 * Ng * C;
@@ -946,20 +974,20 @@ ConvPlan conv_plan(const ConvOrder &ord, int nimg, int h, int w, int C, int N, i
 
 // The order and plan of a shape: the search takes a few microseconds, more
 // than a launch, so each thread keeps the last few dozen shapes' results.
-std::pair<ConvOrder, ConvPlan> conv_lookup(int nimg, int h, int w, int C, int N) {
+std::pair<ConvOrder, ConvPlan> conv_lookup(int nimg, int h, int w, int C, int N, bool one_group) {
     struct Entry {
-        int key[6];
+        int key[7];
         ConvOrder ord;
         ConvPlan plan;
     };
     thread_local Entry cache[64] = {};
-    const int key[6] = {nimg, h, w, C, N, sm_count()};
+    const int key[7] = {nimg, h, w, C, N, one_group, sm_count()};
     uint32_t hash = 2166136261u;
     for (int k : key) hash = (hash ^ (uint32_t)k) * 16777619u;
     Entry &e = cache[(hash >> 16 ^ hash) & 63];
     if (std::memcmp(e.key, key, sizeof(key)) != 0) {
         const ConvOrder ord = conv_order(C, N, w);
-        e.plan = conv_plan(ord, nimg, h, w, C, N, key[5]);
+        e.plan = conv_plan(ord, nimg, h, w, C, N, key[6], one_group);
         e.ord = ord;
         std::memcpy(e.key, key, sizeof(key));
     }
@@ -978,7 +1006,7 @@ void conv3x3_check(int C, int N) {
 // transposed per tap, optional ReLU mask of the layer below).
 void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const float *bias, const __nv_bfloat16 *mask,
                     __nv_bfloat16 *out, float *out_f32, int *err, int nimg, int h, int w, int C, int N, bool flip,
-                    bool relu, cudaStream_t s) {
+                    bool relu, cudaStream_t s, const ConvExtra &x) {
     conv3x3_check(C, N);
     const int64_t P = (int64_t)nimg * h * w;
     CRT_CHECK(nimg > 0 && h > 0 && w > 0 && P < (1LL << 31), CRT_ERR_INVALID, "conv3x3: bad image size");
@@ -988,7 +1016,7 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
                   (!out_f32 || (reinterpret_cast<uintptr_t>(out_f32) & 3) == 0) &&
                   (!mask || (reinterpret_cast<uintptr_t>(mask) & 15) == 0),
               CRT_ERR_INVALID, "conv3x3: output and mask must be 16-byte aligned");
-    const auto [ord, pl] = conv_lookup(nimg, h, w, C, N);
+    const auto [ord, pl] = conv_lookup(nimg, h, w, C, N, x.filtered != nullptr);
     ConvArgs a;
     a.bias = bias;
     a.mask = mask;
@@ -1014,6 +1042,11 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
     a.flip = flip ? 1 : 0;
     a.relu = relu ? 1 : 0;
     a.resident = pl.resident;
+    a.x = x;
+    CRT_CHECK(!x.filtered || (C == 32 && N == 32 && ord.KCo == 32 && pl.groups == 1 && !relu && !flip),
+              CRT_ERR_INVALID, "conv3x3: the filter follows a 32 -> 32 layer");
+    CRT_CHECK(!x.out2 || ((reinterpret_cast<uintptr_t>(x.out2) | (uintptr_t)x.out2_pitch * 2) & 31) == 0,
+              CRT_ERR_INVALID, "conv3x3: the second output must be 32-byte aligned");
     a.vec32 = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
     a.vec_f32 = (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0;
     const int RB = 2 * pl.kc;
@@ -1045,7 +1078,8 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
     using Kfn = void (*)(CUtensorMap, CUtensorMap, ConvArgs, int);
     const Kfn kfns[2][3] = {{k_conv3x3<1, false>, k_conv3x3<2, false>, k_conv3x3<4, false>},
                             {k_conv3x3<1, true>, k_conv3x3<2, true>, k_conv3x3<4, true>}};
-    const Kfn kfn = kfns[ord.rows_outer ? 1 : 0][ord.KCo == 16 ? 0 : ord.KCo == 32 ? 1 : 2];
+    const Kfn kfn = x.filtered ? k_conv3x3<2, false, true>
+                               : kfns[ord.rows_outer ? 1 : 0][ord.KCo == 16 ? 0 : ord.KCo == 32 ? 1 : 2];
     CRT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kfn<<<pl.grid, kConvThreads, smem, s>>>(map_in, map_w, a, pl.kc == 64 ? 6 : pl.kc == 32 ? 5 : 4);
     CRT_CUDA(cudaGetLastError());

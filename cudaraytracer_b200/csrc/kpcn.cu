@@ -21,6 +21,7 @@
 //
 // Loss: relMSE = mean over pixels and RGB of (out - ref)^2 / (ref^2 + 0.01).
 #include "api_internal.h"
+#include "kpcn_filter.cuh"
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -33,7 +34,6 @@ namespace {
 
 constexpr int kLayers = 11;
 constexpr int kFeat = 16;
-constexpr int kTaps5 = 25;
 constexpr int kOutC = 32;
 constexpr float kRelEps = 0.01f;
 
@@ -79,33 +79,6 @@ __global__ void k_avgpool2(const __nv_bfloat16 *in, __nv_bfloat16 *out, int n, i
         for (int k = 0; k < 8; ++k) s[k] *= 0.25f;
         store8(out + q * C + g * 8, s);
     }
-}
-
-// out[p] = concat(up2(low)[p] (Ca), skip[p] (Cb)), 8 channels (16 B) per
-// thread step; index arithmetic in I (32-bit whenever the element count
-// allows: the divisions are most of the work).
-template <class I>
-__device__ __forceinline__ void up_concat(const __nv_bfloat16 *low, const __nv_bfloat16 *skip, __nv_bfloat16 *out,
-                                          int n, int h, int w, int Ca, int Cb) {
-    const int C = Ca + Cb, G = C / 8;
-    const I total = (I)n * h * w * G;
-    for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
-        const int g = (int)(i % G);
-        const I p = i / G;
-        const int x = (int)(p % w), y = (int)((p / w) % h), b = (int)(p / ((I)w * h));
-        const __nv_bfloat16 *src = g * 8 < Ca
-                                       ? low + (((int64_t)b * (h / 2) + y / 2) * (w / 2) + x / 2) * Ca + g * 8
-                                       : skip + (int64_t)p * Cb + (g * 8 - Ca);
-        *reinterpret_cast<uint4 *>(out + (int64_t)p * C + g * 8) = *reinterpret_cast<const uint4 *>(src);
-    }
-}
-
-__global__ void k_up_concat(const __nv_bfloat16 *low, const __nv_bfloat16 *skip, __nv_bfloat16 *out, int n, int h,
-                            int w, int Ca, int Cb) {
-    if ((int64_t)n * h * w * ((Ca + Cb) / 8) < (int64_t)INT32_MAX - (int64_t)gridDim.x * blockDim.x)
-        up_concat<int>(low, skip, out, n, h, w, Ca, Cb);
-    else
-        up_concat<int64_t>(low, skip, out, n, h, w, Ca, Cb);
 }
 
 // Adjoint of up2 on the first Ca channels of gcat: glow[q] = sum of the 2x2
@@ -234,11 +207,9 @@ __global__ void k_features(FeatureArgs a) {
     }
 }
 
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
-
-// Softmax over the 25 logits of one pixel (its 32-float row, 16-byte
-// aligned), weights in w. The row is read as 7 float4 loads (28 floats),
-// not 25 scalar loads that each touch a sector per lane.
+// The filter weights from a pixel's logits (its 32-float row, 16-byte
+// aligned). The row is read as 7 float4 loads (28 floats), not 25 scalar
+// loads that each touch a sector per lane.
 __device__ __forceinline__ void filter_weights(const float *logits, float (&w)[kTaps5]) {
     float l[28];
     const float4 *lp = reinterpret_cast<const float4 *>(logits);
@@ -250,39 +221,7 @@ __device__ __forceinline__ void filter_weights(const float *logits, float (&w)[k
         l[4 * j + 2] = v.z;
         l[4 * j + 3] = v.w;
     }
-    float mx = l[0];
-#pragma unroll
-    for (int k = 1; k < kTaps5; ++k) mx = fmaxf(mx, l[k]);
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < kTaps5; ++k) {
-        w[k] = expf(l[k] - mx);
-        s += w[k];
-    }
-    const float inv = 1.f / s;
-#pragma unroll
-    for (int k = 0; k < kTaps5; ++k) w[k] *= inv;
-}
-
-// out[p] = sum_k w_k(p) * noisy[clamp(p + off5(k))].
-__global__ void k_apply_filter(const float *logits, const float4 *noisy, float4 *out, int n, int h, int w) {
-    const int64_t P = (int64_t)n * h * w;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < P; p += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(p % w), y = (int)((p / w) % h);
-        const int64_t base = p - (int64_t)y * w - x;
-        float wt[kTaps5];
-        filter_weights(logits + p * kOutC, wt);
-        float r = 0.f, g = 0.f, b = 0.f;
-#pragma unroll
-        for (int k = 0; k < kTaps5; ++k) {
-            const int sy = clampi(y + k / 5 - 2, 0, h - 1), sx = clampi(x + k % 5 - 2, 0, w - 1);
-            const float4 v = noisy[base + (int64_t)sy * w + sx];
-            r += wt[k] * v.x;
-            g += wt[k] * v.y;
-            b += wt[k] * v.z;
-        }
-        out[p] = make_float4(r, g, b, 0.f);
-    }
+    softmax25(l, w);
 }
 
 // Loss and its gradient w.r.t. the logits (BF16, 32 channels, 25..31 zero).
@@ -389,6 +328,7 @@ struct crt_kpcn {
     __nv_bfloat16 *act[kLayers] = {};
     __nv_bfloat16 *pool0 = nullptr, *pool1 = nullptr, *cat1 = nullptr, *cat0 = nullptr;
     float *logits = nullptr;
+    bool logits_stored = false;  // logits holds the last forward's
     float *loss = nullptr;
     // gradient buffers
     __nv_bfloat16 *gl = nullptr, *ga = nullptr, *gb = nullptr, *gcat = nullptr, *gpool = nullptr, *gsk = nullptr;
@@ -447,28 +387,46 @@ struct crt_kpcn {
         cap_px = P0;
     }
     void conv(int i, const __nv_bfloat16 *in, int ln, int lh, int lw, __nv_bfloat16 *out, float *out_f32,
-              cudaStream_t s) {
+              cudaStream_t s, const ConvExtra &x = {}) {
         conv3x3_launch(in, L[i].wb, params + L[i].boff, nullptr, out, out_f32, ctx->d_err, ln, lh, lw, L[i].cin,
-                       L[i].cout, false, L[i].relu, s);
+                       L[i].cout, false, L[i].relu, s, x);
     }
-    void forward(const __nv_bfloat16 *feat, cudaStream_t s) {
+    // The concatenated inputs of d1a and d0a are written by the layers they
+    // come from: the skip layer's epilogue stores its pixels a second time,
+    // the lower layer's stores each pixel at its four places. (Separate
+    // upsample-and-concatenate passes took 197 us of a 1920 x 1080 frame.)
+    // With noisy and out the output layer applies the filter in its epilogue
+    // and its logits are not stored (265 MB written and read again, and 106 us
+    // for the filter pass); else they are.
+    void forward(const __nv_bfloat16 *feat, const float4 *noisy, float4 *out, cudaStream_t s) {
         const int h1 = h / 2, w1 = w / 2, h2 = h / 4, w2 = w / 4;
         conv(E0A, feat, n, h, w, act[E0A], nullptr, s);
-        conv(E0B, act[E0A], n, h, w, act[E0B], nullptr, s);
+        conv(E0B, act[E0A], n, h, w, act[E0B], nullptr, s, ConvExtra{cat0 + 64, 96, false, nullptr, nullptr});
         k_avgpool2<<<grid_for((int64_t)n * h1 * w1 * 4), 256, 0, s>>>(act[E0B], pool0, n, h, w, 32);
         conv(E1A, pool0, n, h1, w1, act[E1A], nullptr, s);
-        conv(E1B, act[E1A], n, h1, w1, act[E1B], nullptr, s);
+        conv(E1B, act[E1A], n, h1, w1, act[E1B], nullptr, s, ConvExtra{cat1 + 96, 160, false, nullptr, nullptr});
         k_avgpool2<<<grid_for((int64_t)n * h2 * w2 * 8), 256, 0, s>>>(act[E1B], pool1, n, h1, w1, 64);
         conv(E2A, pool1, n, h2, w2, act[E2A], nullptr, s);
-        conv(E2B, act[E2A], n, h2, w2, act[E2B], nullptr, s);
-        k_up_concat<<<grid_for((int64_t)n * h1 * w1 * 20), 256, 0, s>>>(act[E2B], act[E1B], cat1, n, h1, w1, 96, 64);
+        conv(E2B, act[E2A], n, h2, w2, act[E2B], nullptr, s, ConvExtra{cat1, 160, true, nullptr, nullptr});
         conv(D1A, cat1, n, h1, w1, act[D1A], nullptr, s);
-        conv(D1B, act[D1A], n, h1, w1, act[D1B], nullptr, s);
-        k_up_concat<<<grid_for((int64_t)n * h * w * 12), 256, 0, s>>>(act[D1B], act[E0B], cat0, n, h, w, 64, 32);
+        conv(D1B, act[D1A], n, h1, w1, act[D1B], nullptr, s, ConvExtra{cat0, 96, true, nullptr, nullptr});
         conv(D0A, cat0, n, h, w, act[D0A], nullptr, s);
         conv(D0B, act[D0A], n, h, w, act[D0B], nullptr, s);
-        conv(OUT, act[D0B], n, h, w, nullptr, logits, s);
+        if (out)
+            conv(OUT, act[D0B], n, h, w, nullptr, nullptr, s, ConvExtra{nullptr, 0, false, noisy, out});
+        else
+            conv(OUT, act[D0B], n, h, w, nullptr, logits, s);
+        logits_stored = out == nullptr;
         CRT_CUDA(cudaGetLastError());
+    }
+    // The logits of the last forward, computed again from its last activation
+    // where it went on to the filter (before the parameters change, or for
+    // the debug tensor; the device is idle).
+    void store_logits() {
+        if (logits_stored || n == 0) return;
+        conv(OUT, act[D0B], n, h, w, nullptr, logits, ctx->stream);
+        CRT_CUDA(cudaStreamSynchronize(ctx->stream));
+        logits_stored = true;
     }
     // Gradients of layer i given the pre-activation output gradient g (BF16):
     // dW, db; and, when gin != null, the input gradient (masked by `mask`).
@@ -597,6 +555,7 @@ extern "C" crt_status crt_kpcn_set_params(crt_kpcn *k, const float *host) {
         CRT_CHECK(k && host, CRT_ERR_INVALID, "crt_kpcn_set_params: null argument");
         CRT_CUDA(cudaSetDevice(k->ctx->device));
         CRT_CUDA(cudaDeviceSynchronize());
+        k->store_logits();
         CRT_CUDA(cudaMemcpy(k->params, host, k->nparams * sizeof(float), cudaMemcpyHostToDevice));
         k->refresh_bf16(k->ctx->stream);
         CRT_CUDA(cudaStreamSynchronize(k->ctx->stream));
@@ -637,10 +596,7 @@ extern "C" crt_status crt_kpcn_forward(crt_kpcn *k, int32_t n, int32_t h, int32_
         CRT_CUDA(cudaSetDevice(k->ctx->device));
         cudaStream_t s = stream ? (cudaStream_t)stream : k->ctx->stream;
         k->ensure(n, h, w);
-        k->forward((const __nv_bfloat16 *)d_features, s);
-        k_apply_filter<<<grid_for((int64_t)n * h * w), 256, 0, s>>>(k->logits, (const float4 *)d_noisy,
-                                                                      (float4 *)d_out, n, h, w);
-        CRT_CUDA(cudaGetLastError());
+        k->forward((const __nv_bfloat16 *)d_features, (const float4 *)d_noisy, (float4 *)d_out, s);
     });
 }
 
@@ -655,7 +611,7 @@ extern "C" crt_status crt_kpcn_train_step(crt_kpcn *k, int32_t n, int32_t h, int
         cudaStream_t s = stream ? (cudaStream_t)stream : k->ctx->stream;
         k->ensure(n, h, w);
         const __nv_bfloat16 *feat = (const __nv_bfloat16 *)d_features;
-        k->forward(feat, s);
+        k->forward(feat, nullptr, nullptr, s);
         const int64_t P = (int64_t)n * h * w;
         CRT_CUDA(cudaMemsetAsync(k->loss, 0, sizeof(float), s));
         k_filter_loss_grad<<<grid_for(P), 256, 0, s>>>(k->logits, (const float4 *)d_noisy, (const float4 *)d_target,
@@ -703,6 +659,7 @@ extern "C" crt_status crt_kpcn_debug_tensor(crt_kpcn *k, int32_t which, void *ho
             src = k->act[which];
             sz = P[which] * k->L[which].cout * 2;
         } else if (which == 10) {
+            k->store_logits();
             src = k->logits;
             sz = P0 * kOutC * 4;
         } else if (which == 11) {
