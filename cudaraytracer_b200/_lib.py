@@ -278,6 +278,8 @@ _SIGS = {
 def lib() -> C.CDLL:
     """Loads libcrt.so (raises if it has not been built)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):

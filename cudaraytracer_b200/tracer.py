@@ -17,6 +17,7 @@ pipelined in chunks) or CUDA torch tensors (device path, no copies).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import numpy as np
 
@@ -31,11 +32,25 @@ def _torch_stream(device, stream=None) -> int:
     """cudaStream_t of `stream` (or torch's current stream). Torch's default
     stream has handle 0, which the C ABI reads as "the context's own stream",
     so it is passed as cudaStreamLegacy (1) instead."""
+    if stream is None and device.index is not None:
+        # the handle alone: building torch's Stream object around it takes
+        # longer than the launch of a small batch
+        s = _raw_stream()(device.index)
+    else:
+        import torch
+
+        s = stream if stream is not None else torch.cuda.current_stream(device).cuda_stream
+        s = int(getattr(s, "cuda_stream", s))
+    return s if s != 0 else 1
+
+
+@functools.lru_cache(maxsize=None)
+def _raw_stream():
+    """torch's current stream handle by device index."""
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream(device).cuda_stream
-    s = int(getattr(s, "cuda_stream", s))
-    return s if s != 0 else 1
+    fn = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return fn if fn is not None else lambda index: torch.cuda.current_stream(index).cuda_stream
 
 
 class Context:
