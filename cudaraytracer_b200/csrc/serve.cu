@@ -22,6 +22,7 @@
 #include "path.cuh"
 #include "path_loop.cuh"
 #include <algorithm>
+#include <climits>
 #include <deque>
 #include <map>
 #include <unordered_map>
@@ -505,7 +506,10 @@ struct crt_server {
         const ShadeOrder ord{wf.order, (int)wf.cap, nullptr};  // ks_extend takes each path's scene's classes
         ks_raygen<<<(n + 255) / 256, 256, 0, stream>>>(d_reqs, ds, nseg, n, q[0], wf.counters);
         const int smem = stage_traversal_env();
-        const int b_paths = path_start(smem, n);
+        // A pass too large for the path kernel's first two rules keeps the
+        // stages: with a scene and a request per lane it gains nothing there
+        // (4M-path passes over Cornell boxes, 12.37 against 12.29 ms).
+        const int b_paths = n <= kPathFromSecond ? path_start(smem, n) : INT_MAX;
         for (int b = 0; b < max_b; ++b) {
             const int in = b & 1, out = 1 - in;
             if (b >= b_paths) {
