@@ -407,10 +407,12 @@ constexpr int kTinyVariant = 11;
 constexpr int kFlatVariant = 14;
 constexpr int kVoteVariant = 15;
 // Smaller batches leave lanes without a second ray, and a vote only delays
-// the lanes it passes over: at 20,001 rays on a 5,120-triangle field the
-// lane-refill kernels take 22 / 49 us, voting 25 / 57; even at 200,000 (57 /
-// 132 against 59 / 131), ahead at a million (137 / 557 against 113 / 441).
-constexpr int64_t kVoteMinRays = 160 << 10;
+// the lanes it passes over. Closest + shadow, cold L2, lane refill against
+// voting, us: 20K triangles 168 / 178 at 260,000 rays, 195 / 191 at 320,000,
+// 253 / 225 at 500,000; 82K triangles 184 / 189 at 150,000, 229 / 226 at
+// 260,000, 264 / 249 at 320,000; 1.3M triangles 315 / 323 at 150,000,
+// 414 / 374 at 260,000. The line is where the smallest of them turns.
+constexpr int64_t kVoteMinRays = 288 << 10;
 
 static int traversal_variant(const BvhView &bvh, int64_t n) {
     const char *e = getenv("CRT_TRAVERSAL");
