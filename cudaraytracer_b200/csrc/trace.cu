@@ -417,11 +417,12 @@ constexpr int kFlatVariant = 14;
 constexpr int kVoteVariant = 15;
 // Smaller batches leave lanes without a second ray, and a vote only delays
 // the lanes it passes over. Closest + shadow, cold L2, lane refill against
-// voting, us: 20K triangles 168 / 178 at 260,000 rays, 195 / 191 at 320,000,
-// 253 / 225 at 500,000; 82K triangles 184 / 189 at 150,000, 229 / 226 at
-// 260,000, 264 / 249 at 320,000; 1.3M triangles 315 / 323 at 150,000,
-// 414 / 374 at 260,000. The line is where the smallest of them turns.
-constexpr int64_t kVoteMinRays = 288 << 10;
+// voting, us: 20K triangles 173 / 174 at 260,000 rays, 187 / 189 at 320,000,
+// 210 / 207 at 400,000, 247 / 227 at 500,000; 82K triangles 203 / 202 at
+// 200,000, 310 / 293 at 400,000; 1.3M triangles 305 / 323 at 150,000,
+// 391 / 379 at 260,000, 499 / 453 at 400,000. The line is where the smallest
+// of them turns.
+constexpr int64_t kVoteMinRays = 352 << 10;
 
 static int traversal_variant(const BvhView &bvh, int64_t n) {
     const char *e = getenv("CRT_TRAVERSAL");

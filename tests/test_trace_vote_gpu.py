@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 31, 33, 63, 64, 65, 577, 4097, 200_003, 300_007]
+SIZES = [1, 31, 33, 63, 64, 65, 577, 4097, 200_003, 400_009]
 
 
 @pytest.mark.parametrize("spheres,level", [(1, 0), (2, 2), (16, 4)])
