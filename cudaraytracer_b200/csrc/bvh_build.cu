@@ -702,10 +702,11 @@ __global__ void k_flat(const float4 *tris, int n, float4 *flat) {
                              e1.x, e1.y, e1.z, f2.y,         f1.x, f1.y, f1.z, f2.z};
         float *p = reinterpret_cast<float *>(flat) + 32 * (k / 2) + (k & 1);
         for (int j = 0; j < 16; ++j) p[2 * j] = r[j];
-        // an odd scene's last record has no second triangle: T = -1 there
-        // (det = 0 and a zero v0 would leave it a candidate)
+        // an odd scene's last record has no second triangle: T is NaN there,
+        // which no margin lets pass, infinite ones included (as a candidate
+        // its slot would lie past the triangles)
         if (k == n - 1 && !(k & 1))
-            for (int j = 0; j < 16; ++j) p[2 * j + 1] = j == 3 ? -1e30f : 0.f;
+            for (int j = 0; j < 16; ++j) p[2 * j + 1] = j == 3 ? nanf("") : 0.f;
         s_e[k] = fmaxf(fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z), fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z));
         s_v[k] = fabsf(v0.x) + fabsf(v0.y) + fabsf(v0.z);
     }
