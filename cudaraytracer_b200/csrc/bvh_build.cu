@@ -707,19 +707,22 @@ __global__ void k_flat(const float4 *tris, int n, float4 *flat) {
         // its slot would lie past the triangles)
         if (k == n - 1 && !(k & 1))
             for (int j = 0; j < 16; ++j) p[2 * j + 1] = j == 3 ? nanf("") : 0.f;
-        s_e[k] = fmaxf(fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z), fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z));
+        // (fmaxf drops a NaN: one edge's would hide behind the other's length)
+        const float l1 = fabsf(e1.x) + fabsf(e1.y) + fabsf(e1.z), l2 = fabsf(e2.x) + fabsf(e2.y) + fabsf(e2.z);
+        s_e[k] = l1 < INFINITY ? fmaxf(l1, l2 < INFINITY ? l2 : INFINITY) : INFINITY;
         s_v[k] = fabsf(v0.x) + fabsf(v0.y) + fabsf(v0.z);
     }
     __syncthreads();
     if (k == 0) {
         float e = 0.f, v = 0.f;
+        bool finite = true;
         for (int i = 0; i < n; ++i) {
             e = fmaxf(e, s_e[i]);
             v = fmaxf(v, s_v[i]);
+            finite = finite && s_e[i] < INFINITY && s_v[i] < INFINITY;
         }
-        // NaN vertices must not pass for small ones
-        for (int i = 0; i < n; ++i)
-            if (!(s_e[i] <= e) || !(s_v[i] <= v)) e = v = INFINITY;
+        // NaN vertices must not pass for small ones: the tree decides
+        if (!finite) e = v = INFINITY;
         flat[8 * ((n + 1) / 2)] = make_float4(e, v, 0.f, 0.f);
     }
 }

@@ -60,3 +60,13 @@ def test_huge_origins(crt_ctx, n):
     r[:, 0:3] *= far
     r[::2, 4:7] = -r[::2, 0:3] / far[::2]  # towards the scene
     check(crt_ctx, soup(n, n), r)
+
+
+@pytest.mark.parametrize("comp", [0, 3, 5, 7, 8])
+@pytest.mark.parametrize("n", [16, 21, 32, 63])
+def test_nan_vertices(crt_ctx, n, comp):
+    """A triangle with one NaN coordinate, of any of its vertices: the tree
+    accepts it with t = NaN or not by the order of its nodes."""
+    tris = soup(n, 7 * n)
+    tris[n // 3, comp] = np.nan
+    check(crt_ctx, tris, random_rays(1 << 14, n + comp))
