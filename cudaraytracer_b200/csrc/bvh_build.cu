@@ -721,8 +721,10 @@ __global__ void k_flat(const float4 *tris, int n, float4 *flat) {
             v = fmaxf(v, s_v[i]);
             finite = finite && s_e[i] < INFINITY && s_v[i] < INFINITY;
         }
-        // NaN vertices must not pass for small ones: the tree decides
-        if (!finite) e = v = INFINITY;
+        // NaN vertices must not pass for small ones, and the margins must bound
+        // the roundings of products of lengths: else the tree decides (flat.cuh)
+        v = fmaxf(v, 1e-12f);
+        if (!finite || e < 1e-10f || e > 1e10f) e = v = INFINITY;
         flat[8 * ((n + 1) / 2)] = make_float4(e, v, 0.f, 0.f);
     }
 }

@@ -65,10 +65,11 @@ template <bool kEarlyExit>
 __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView &bvh, V3 o, V3 d, float tmin,
                                                 float tmax, float t_exit = 0.f) {
     const int n = bvh.num_tris, pairs = (n + 1) >> 1;
-    const float4 sc = rec[8 * pairs];  // E, max |v0|
+    const float4 sc = rec[8 * pairs];  // E, max |v0|, in the ranges k_flat keeps them in
     const float d1 = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
     const float s1n = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + sc.y;
-    const float md = 2e-6f * d1 * sc.x * sc.x, mt = 2e-6f * s1n * sc.x * sc.x, mu = 2e-6f * d1 * sc.x * s1n;
+    const float sd = s1n * d1;
+    const float md = 2e-6f * d1 * sc.x * sc.x, mt = 2e-6f * s1n * sc.x * sc.x, mu = 2e-6f * sc.x * sd;
     const float mw = 2.f * (mu + md);
     const float mx = o.y * d.z - o.z * d.y, my = o.z * d.x - o.x * d.z, mz = o.x * d.y - o.y * d.x;
     const F2 dx = f2(d.x, d.x), dy = f2(d.y, d.y), dz = f2(d.z, d.z);
@@ -100,8 +101,10 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
     hit.slot = -1;
     hit.b1 = hit.b2 = 0.f;
     float best = INFINITY, second = INFINITY, det_b = 1.f;
-    // margins out of range (huge or non-finite rays): the tree decides
-    bool odd = !(md < 1e30f && mt < 1e30f && mu < 1e30f), clear = false;
+    // Products beyond the floats, or so small that their roundings are not
+    // relative (huge, tiny or non-finite rays; k_flat keeps 1e-10 <= E <= 1e10
+    // and S >= 1e-12, so no margin falls below 1e-40): the tree decides.
+    bool odd = !(md + mt + mu + sd < 1e30f) || !(d1 > 1e-12f), clear = false;
     while (cand[0] | cand[1]) {
         int slot;
         if (cand[0]) {

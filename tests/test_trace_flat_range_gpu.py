@@ -70,3 +70,42 @@ def test_nan_vertices(crt_ctx, n, comp):
     tris = soup(n, 7 * n)
     tris[n // 3, comp] = np.nan
     check(crt_ctx, tris, random_rays(1 << 14, n + comp))
+
+
+@pytest.mark.parametrize("n", [2, 13, 32, 63])
+@pytest.mark.parametrize("exponent", [-46, -43, -40, -34, -20, 20, 34])
+def test_scaled_scenes(crt_ctx, n, exponent):
+    """A scene and its rays scaled by a power of two: products of three
+    lengths leave the range of normal floats."""
+    from cudaraytracer_b200 import scenes
+
+    s = np.float32(2.0 ** exponent)
+    tris, r = soup(n, 100 + n), random_rays(1 << 16, n)
+    q = scenes.random_shadow_queries(tris, 1 << 14, seed=n)
+    t = tris.reshape(-1, 3, 3)
+    k, w = np.arange(1 << 14) % n, np.random.default_rng(n).dirichlet((1, 1, 1), 1 << 14)
+    r[:1 << 14, 0:3] = np.einsum("nk,nkc->nc", w, t[k])  # from points of triangles
+    r[:, 0:3] *= s
+    q[:, 0:3] *= s
+    q[:, 6:9] *= s
+    check(crt_ctx, tris * s, r, q)
+    r[:, 4:7] *= np.float32(2.0 ** -30)
+    check(crt_ctx, tris * s, r, q)
+
+
+@pytest.mark.parametrize("n", [2, 3, 32])
+def test_products_beyond_the_largest_float(crt_ctx, n):
+    """Origin times direction overflows where the triangle test's own
+    products do not: rays along the diagonals into triangles around them."""
+    d, s = 1e16, 5e23
+    tris, r = [], np.zeros((64, 8), np.float32)
+    for k in range(max(n, 64)):
+        sx, sy, e = (-1) ** (k & 1), (-1) ** (k >> 1 & 1), 1e-6 / (1 + k)
+        if k < n:  # facing the origin of the rays of this diagonal
+            tris.append([[0, 0, -e / 4], [0, 0, e], [e * sy, -e * sx, -e / 4]])
+        if k < 64:
+            r[k, 0:3] = np.array([sx, sy, 0]) * s * 2.0 ** -(k >> 2)
+            r[k, 4:7] = np.array([-sx, -sy, 0]) * d
+    r[:, 7] = 1e8
+    prims = check(crt_ctx, np.array(tris, np.float32).reshape(n, 9), r)
+    assert (prims >= 0).any()
