@@ -143,7 +143,8 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
         }
     }
     if (hit.slot >= 0) {
-        const float gap = mt / det_b + 2e-6f * best;  // rounding of t
+        // rounding of t = T / det: T's, det's and the quotient's
+        const float gap = (mt + md * best) / det_b + 2e-6f * best;
         if (best > tmax + gap) {  // beyond the caller's bound, clearly: no hit
             hit.slot = -1;
             hit.b1 = hit.b2 = 0.f;

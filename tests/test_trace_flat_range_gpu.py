@@ -109,3 +109,26 @@ def test_products_beyond_the_largest_float(crt_ctx, n):
     r[:, 7] = 1e8
     prims = check(crt_ctx, np.array(tris, np.float32).reshape(n, 9), r)
     assert (prims >= 0).any()
+
+
+@pytest.mark.parametrize("tilt", [0.0, 1e-6, 1e-3])
+@pytest.mark.parametrize("n", [12, 33, 64])
+def test_fans_around_the_origin(crt_ctx, n, tilt):
+    """Long, nearly coplanar triangles that share a vertex close to grazing
+    rays: the determinants cancel, and t's error is det's."""
+    rng = np.random.default_rng(n)
+    a, da, m, length = rng.uniform(0, 2 * np.pi, n), rng.uniform(0.01, 1.0, n), 1 << 17, 100.0
+
+    def far(a):
+        r = length * rng.uniform(0.5, 1, n)
+        return np.stack([r * np.cos(a), r * np.sin(a), r * tilt * rng.normal(size=n)], 1)
+
+    t = np.zeros((n, 3, 3))
+    t[:, 1], t[:, 2] = far(a), far(a + da)
+    t[::2, 1:] = t[::2, :0:-1]  # both facings
+    r = np.zeros((m, 8), np.float32)
+    b, c = rng.uniform(0, 2 * np.pi, m), 10 ** rng.uniform(-7, -1, m) * rng.choice([-1, 1], m)
+    r[:, 0:3] = rng.normal(size=(m, 3)) * 10 ** rng.uniform(-8, -2, (m, 1))
+    r[:, 4:7], r[:, 7] = np.stack([np.cos(b), np.sin(b), c], 1), 1e8
+    prims = check(crt_ctx, t.reshape(n, 9).astype(np.float32), r)
+    assert (prims >= 0).mean() > 0.05
