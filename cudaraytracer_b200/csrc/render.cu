@@ -770,6 +770,8 @@ __global__ void __launch_bounds__(kPathBlock, kMinBlocks) k_paths(SceneView s, S
 
 int path_start(int mode, int n) {
     if (mode != kStageLocal && mode != kStageRefill) return INT_MAX;
+    const char *e = getenv("CRT_PATH_KERNEL");  // 0: the stage kernels throughout
+    if (e && e[0] == '0') return INT_MAX;
     return n <= kPathFromStart ? 0 : n <= kPathFromSecond ? 1 : 2;
 }
 
@@ -871,7 +873,8 @@ int render_samples(const SceneView &view, const CameraState &cam, const RenderPa
         sp.pixels = pixels;
         k_raygen<<<(n + 255) / 256, 256, 0, stream>>>(cv, sp, n, q[0], wf.counters);
         ++launches;
-        const int b_paths = path_start(smem, n);
+        // (a register cap asked for the shade stage keeps the stages)
+        const int b_paths = mb ? INT_MAX : path_start(smem, n);
         for (int b = 0; b < rp.max_bounces; ++b) {
             int in = b & 1, out = 1 - in;
             sp.bounce = b;

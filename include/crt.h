@@ -202,16 +202,18 @@ typedef struct crt_render_params {
     int32_t spp_per_pass;     /* samples per wavefront of crt_render*; 0 = automatic */
     int32_t paths_per_pass;   /* paths per wavefront of crt_render_views; 0 = 8M */
     int32_t stage_block;      /* threads per block of the extend/shade/shadow wavefront stages
-                                 (64, 128 or 256); 0 = 128 */
+                                 (64, 128 or 256); 0 = 128. Bounces that the path kernel takes
+                                 (below) do not depend on it */
     int32_t stage_traversal;  /* BVH traversal of the extend and shadow stages: 0 = library
                                  default, else one of CRT_STAGE_* below */
 } crt_render_params;
 
 /* crt_render_params.stage_traversal: where each path's traversal stack lives
  * and which node layout it reads. With DEFAULT, LOCAL and REFILL the late
- * bounces of a pass, and all bounces of a small one, run in one kernel that
- * keeps a path per lane (local stack, float nodes); the others keep the
- * stage kernels throughout. */
+ * bounces of a pass, and all bounces of a small one (up to 655,360 paths), run
+ * in the path kernel, which keeps a path per lane (local stack, float nodes);
+ * the others keep the stage kernels throughout, as CRT_PATH_KERNEL=0 in the
+ * environment does in every mode. */
 #define CRT_STAGE_DEFAULT 0       /* CRT_STAGE_TRAVERSAL from the environment, else LOCAL */
 #define CRT_STAGE_LOCAL 1         /* 64-entry stack in local memory, 64 B float nodes */
 #define CRT_STAGE_SHARED 2        /* top 8 entries in shared memory, 64 B float nodes */
