@@ -24,6 +24,7 @@
 #include "api_internal.h"
 #include "tc.cuh"
 #include "kpcn_filter.cuh"
+#include "conv_plan.h"
 #include <algorithm>
 #include <cstring>
 #include <utility>
@@ -36,8 +37,6 @@ namespace {
 constexpr int kBM = 128;           // k_conv3x3_wgrad: (tap, c) rows per tile
 constexpr int kThreads = 128;      // k_conv3x3_wgrad
 constexpr int kConvThreads = 352;  // k_conv3x3, k_conv3x3_wgrad_ring: TMA warp, 2 MMA warps, 8 epilogue warps
-constexpr int kMaxStages = 5;
-constexpr int kMaxSlots = 8;       // TMEM accumulators of k_conv3x3
 constexpr int kStages = 4;         // k_conv3x3_wgrad pipeline depth
 constexpr int kWgradBK = 64;       // k_conv3x3_wgrad: pixels per K step
 
@@ -862,138 +861,6 @@ void encode_map(CUtensorMap *m, const void *ptr, cuuint32_t rank, const cuuint64
     CRT_CHECK(r == CUDA_SUCCESS, CRT_ERR_CUDA, "conv3x3: tensor map encoding failed");
 }
 
-size_t round1k(size_t v) { return (v + 1023) & ~(size_t)1023; }
-
-// The order in which a layer sums its products, a function of its shape
-// only: the MMAs of one output run over channel chunks of KCo channels (all
-// nine taps of a chunk, then the next chunk) or, with rows_outer, over the
-// three tap rows with the chunks inside. BF16 activations round the sums,
-// so a different order would flip roundings layer by layer; the thresholds
-// below keep every shape's order, and with it every output bit, as it was
-// under the tiling they came from (channels as M, 256 pixels as N).
-struct ConvOrder {
-    int KCo;
-    bool rows_outer;
-};
-
-ConvOrder conv_order(int C, int N, int w) {
-    const int np = (N > 128 || w <= 128) ? 128 : 256;
-    const size_t cap = 220 * 1024 - 1024 - 2048 - 8192, wbytes = round1k((size_t)9 * N * C * 2);
-    auto region = [&](int rb) { return round1k((size_t)(np + 2) * rb); };
-    const int kc = C % 64 == 0 ? 64 : C % 32 == 0 ? 32 : 16;
-    if (wbytes + 4 * (C / kc) * region(2 * kc) <= cap) return {kc, C > kc};
-    for (int c : {64, 32, 16})
-        if (C % c == 0 && wbytes + 9 * region(2 * c) <= cap) return {c, false};
-    for (int ns : {4, 3, 2})
-        for (int c : {64, 32, 16})
-            if ((ns >= 3 || c == 16) && C % c == 0 && ns * (3 * region(2 * c) + round1k((size_t)c * 18 * N)) <= cap)
-                return {c, false};
-    throw Error(CRT_ERR_INVALID, "conv3x3: tile does not fit shared memory");
-}
-
-// The tiling of a layer, by a cost model in SM cycles: an MMA of 128 x Ng
-// x 16 reads 4 KB + 32 Ng B of shared memory at 128 B per cycle or
-// multiplies at 4096 MAC per cycle, whichever is longer; a CTA's loads run
-// at about 32 B per cycle; an epilogue group needs about 400 + 10 Ng cycles
-// per tile and there are two; an MMA warp needs about 58 cycles per MMA and
-// 250-300 per tile, and there are two. A block takes the longest of these,
-// and the layer the CTA with the most blocks.
-struct ConvPlan {
-    int Ng, groups, Ws, R, TS, KCs, kc, S, resident, grid;
-    double cost;
-};
-
-// Rows of shared memory that a block's last tile reads past its stage
-// (their results are dropped).
-size_t conv_over_rows(int tiles, int TS, int R, int P) { return (size_t)std::max(0, (tiles - 1) * TS + 130 - R * P); }
-
-// one_group: all output channels in one CTA (the filter needs a pixel's 32).
-ConvPlan conv_plan(const ConvOrder &ord, int nimg, int h, int w, int C, int N, int sms, bool one_group) {
-    ConvPlan best{};
-    best.cost = 1e30;
-    const size_t cap = 227 * 1024 - 1024 - 4096;  // minus base alignment and static shared memory
-    for (int groups = 1; groups <= (one_group ? 1 : N / 16); ++groups) {
-        if (N % (16 * groups)) continue;
-        const int Ng = N / groups;
-        const size_t wall = (size_t)18 * Ng * C;
-        int stride = 32;
-        while (stride < Ng) stride <<= 1;
-        const int slots = std::min(kMaxSlots, 512 / stride);
-        const double mma = 9.0 * (C / 16) * std::max(0.5 * Ng, 34.0 + 0.25 * Ng);
-        const double epi = 0.5 * (400.0 + 10.0 * Ng);
-        for (int KCs : {C, 64, 32, 16}) {
-            if (KCs > C || C % KCs || KCs % ord.KCo || (ord.rows_outer && KCs != C)) continue;
-            const int kc = KCs % 64 == 0 ? 64 : KCs % 32 == 0 ? 32 : 16;
-            const int nst = C / KCs;
-            for (int resident = 1; resident >= 0; --resident) {
-                if (resident && wall > cap) continue;
-                if (!resident && KCs > 64) continue;
-                for (int mode = 0; mode < 3; ++mode) {
-                    // one image row of 128 pixels per tile, or tiles across
-                    // the rows of strips of equal width (at most 254; at
-                    // most 126 for shorter blocks)
-                    const int lim = mode == 1 ? 254 : 126;
-                    const int strips = mode == 0 ? (w + 127) / 128 : (w + lim - 1) / lim;
-                    const int Ws = mode == 0 ? 128 : (w + strips - 1) / strips;
-                    const int P = Ws + 2, TS = mode == 0 ? P : 128;
-                    for (int R : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32}) {
-                        if (R > h && R > 1) break;
-                        const int tiles = mode == 0 ? R : ((R - 1) * P + Ws + 127) / 128;
-                        if (nst > 1 && tiles > slots) break;
-                        const size_t region = round1k((size_t)(R + 2) * P * 2 * kc);
-                        const size_t stage = (KCs / kc) * region + (resident ? 0 : round1k((size_t)18 * Ng * KCs));
-                        const size_t fixed = (resident ? round1k(wall) : 0) + conv_over_rows(tiles, TS, R, P) * 2 * kc;
-                        if (fixed + stage > cap) break;
-                        const int S = (int)std::min<size_t>(kMaxStages, (cap - fixed) / stage);
-                        const int64_t nblk = (int64_t)nimg * strips * ((h + R - 1) / R);
-                        const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(nblk, sms / groups));
-                        const int64_t rounds = (nblk + ctas - 1) / ctas;
-                        const double load = ((double)(R + 2) * P * 2 * C + (resident ? 0.0 : (double)wall)) / 32;
-                        double total;
-                        if (nst == 1) {  // the warps take alternate blocks
-                            const double issue = tiles * (9.0 * (C / 16) * 58 + 300) + 400;
-                            const double pipe = std::max(std::max(tiles * mma, load), tiles * epi);
-                            total = S > 1 || rounds == 1 ? std::max(rounds * pipe, (rounds + 1) / 2 * issue)
-                                                         : rounds * (issue + load + 1000);
-                        } else {  // alternate tiles of each stage
-                            const double issue = (tiles + 1) / 2 * (9.0 * (KCs / 16) * 58 + 250) + 350;
-                            const double stage_t = std::max(std::max(tiles * mma / nst, load / nst), issue);
-                            total = rounds * std::max(nst * (S > 1 ? stage_t : stage_t + load / nst + 1000), tiles * epi);
-                        }
-                        const double cost = total + load / nst + 2 * epi + (resident ? wall / 40.0 : 0.0);
-                        if (cost < best.cost)
-                            best = ConvPlan{Ng, groups, Ws, R, TS, KCs, kc, S, resident, ctas * groups, cost};
-                    }
-                }
-            }
-        }
-    }
-    CRT_CHECK(best.cost < 1e30, CRT_ERR_INVALID, "conv3x3: tile does not fit shared memory");
-    return best;
-}
-
-// The order and plan of a shape: the search takes a few microseconds, more
-// than a launch, so each thread keeps the last few dozen shapes' results.
-std::pair<ConvOrder, ConvPlan> conv_lookup(int nimg, int h, int w, int C, int N, bool one_group) {
-    struct Entry {
-        int key[7];
-        ConvOrder ord;
-        ConvPlan plan;
-    };
-    thread_local Entry cache[64] = {};
-    const int key[7] = {nimg, h, w, C, N, one_group, sm_count()};
-    uint32_t hash = 2166136261u;
-    for (int k : key) hash = (hash ^ (uint32_t)k) * 16777619u;
-    Entry &e = cache[(hash >> 16 ^ hash) & 63];
-    if (std::memcmp(e.key, key, sizeof(key)) != 0) {
-        const ConvOrder ord = conv_order(C, N, w);
-        e.plan = conv_plan(ord, nimg, h, w, C, N, key[6], one_group);
-        e.ord = ord;
-        std::memcpy(e.key, key, sizeof(key));
-    }
-    return {e.ord, e.plan};
-}
-
 }  // namespace
 
 void conv3x3_check(int C, int N) {
@@ -1016,7 +883,8 @@ void conv3x3_launch(const __nv_bfloat16 *in, const __nv_bfloat16 *wgt, const flo
                   (!out_f32 || (reinterpret_cast<uintptr_t>(out_f32) & 3) == 0) &&
                   (!mask || (reinterpret_cast<uintptr_t>(mask) & 15) == 0),
               CRT_ERR_INVALID, "conv3x3: output and mask must be 16-byte aligned");
-    const auto [ord, pl] = conv_lookup(nimg, h, w, C, N, x.filtered != nullptr);
+    thread_local ConvPlans plans;
+    const auto [ord, pl] = plans.get(nimg, h, w, C, N, x.filtered != nullptr, sm_count());
     ConvArgs a;
     a.bias = bias;
     a.mask = mask;
