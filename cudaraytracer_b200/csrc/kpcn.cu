@@ -329,6 +329,11 @@ struct crt_kpcn {
     __nv_bfloat16 *pool0 = nullptr, *pool1 = nullptr, *cat1 = nullptr, *cat0 = nullptr;
     float *logits = nullptr;
     bool logits_stored = false;  // logits holds the last forward's
+    // the output layer's parameters at the last forward, where set_params has
+    // replaced them since and the logits are not stored
+    __nv_bfloat16 *out_wb = nullptr;
+    float *out_bias = nullptr;
+    bool out_kept = false;
     float *loss = nullptr;
     // gradient buffers
     __nv_bfloat16 *gl = nullptr, *ga = nullptr, *gb = nullptr, *gcat = nullptr, *gpool = nullptr, *gsk = nullptr;
@@ -336,7 +341,8 @@ struct crt_kpcn {
 
     ~crt_kpcn() {
         free_buffers();
-        for (void *p : {(void *)params, (void *)grads, (void *)adam_m, (void *)adam_v, (void *)wbuf})
+        for (void *p : {(void *)params, (void *)grads, (void *)adam_m, (void *)adam_v, (void *)wbuf, (void *)out_wb,
+                        (void *)out_bias})
             if (p) cudaFree(p);
     }
     void free_buffers() {
@@ -417,14 +423,24 @@ struct crt_kpcn {
         else
             conv(OUT, act[D0B], n, h, w, nullptr, logits, s);
         logits_stored = out == nullptr;
+        out_kept = false;
         CRT_CUDA(cudaGetLastError());
     }
+    // Before the parameters change: keeps the output layer's for store_logits.
+    void keep_out_params() {
+        if (logits_stored || out_kept || n == 0) return;
+        CRT_CUDA(cudaMemcpy(out_wb, L[OUT].wb, (size_t)9 * L[OUT].cout * L[OUT].cin * sizeof(__nv_bfloat16),
+                            cudaMemcpyDeviceToDevice));
+        CRT_CUDA(cudaMemcpy(out_bias, params + L[OUT].boff, L[OUT].cout * sizeof(float), cudaMemcpyDeviceToDevice));
+        out_kept = true;
+    }
     // The logits of the last forward, computed again from its last activation
-    // where it went on to the filter (before the parameters change, or for
-    // the debug tensor; the device is idle).
+    // and its parameters where it went on to the filter (for the debug
+    // tensor; the device is idle).
     void store_logits() {
         if (logits_stored || n == 0) return;
-        conv(OUT, act[D0B], n, h, w, nullptr, logits, ctx->stream);
+        conv3x3_launch(act[D0B], out_kept ? out_wb : L[OUT].wb, out_kept ? out_bias : params + L[OUT].boff, nullptr,
+                       nullptr, logits, ctx->d_err, n, h, w, L[OUT].cin, L[OUT].cout, false, L[OUT].relu, ctx->stream);
         CRT_CUDA(cudaStreamSynchronize(ctx->stream));
         logits_stored = true;
     }
@@ -497,6 +513,8 @@ extern "C" crt_status crt_kpcn_create(crt_ctx *ctx, uint64_t seed, crt_kpcn **ou
         CRT_CUDA(cudaMalloc(&k->adam_m, off * sizeof(float)));
         CRT_CUDA(cudaMalloc(&k->adam_v, off * sizeof(float)));
         CRT_CUDA(cudaMalloc(&k->wbuf, wbf * sizeof(__nv_bfloat16)));
+        CRT_CUDA(cudaMalloc(&k->out_wb, (size_t)9 * kSpec[OUT].cout * kSpec[OUT].cin * sizeof(__nv_bfloat16)));
+        CRT_CUDA(cudaMalloc(&k->out_bias, kSpec[OUT].cout * sizeof(float)));
         CRT_CUDA(cudaMemset(k->adam_m, 0, off * sizeof(float)));
         CRT_CUDA(cudaMemset(k->adam_v, 0, off * sizeof(float)));
         size_t bo = 0;
@@ -555,7 +573,7 @@ extern "C" crt_status crt_kpcn_set_params(crt_kpcn *k, const float *host) {
         CRT_CHECK(k && host, CRT_ERR_INVALID, "crt_kpcn_set_params: null argument");
         CRT_CUDA(cudaSetDevice(k->ctx->device));
         CRT_CUDA(cudaDeviceSynchronize());
-        k->store_logits();
+        k->keep_out_params();
         CRT_CUDA(cudaMemcpy(k->params, host, k->nparams * sizeof(float), cudaMemcpyHostToDevice));
         k->refresh_bf16(k->ctx->stream);
         CRT_CUDA(cudaStreamSynchronize(k->ctx->stream));
