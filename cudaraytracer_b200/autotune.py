@@ -5,8 +5,10 @@ and placement: a 64-entry stack in local memory or the top 8 entries in
 shared memory; node width: 64 B float child boxes or 32 B 16-bit quantised
 ones) for Scene.render_views, by timing a short probe render of each
 candidate with CUDA events, and caches the choice in a JSON file keyed by
-GPU name, scene triangle count (power-of-two bucket), image size and view
-count. The branching factor stays binary (the 4- and 8-wide collapses
+VERSION (choices made before the kernels changed are not taken over), GPU
+name, scene triangle count (power-of-two bucket), image size and view count.
+With "local" and "refill" the later bounces of a pass run in the path kernel,
+which the block size does not concern. The branching factor stays binary (the 4- and 8-wide collapses
 measured slower). No counterpart in the reference (its wavefront is one
 frame of one view)."""
 from __future__ import annotations
@@ -15,6 +17,9 @@ import json
 import math
 import os
 
+# of what is tuned: raised when the candidates run other kernels than before
+# (2: the path kernel under "local" and "refill")
+VERSION = 2
 DEFAULT_CANDIDATES = (1 << 20, 2 << 20, 4 << 20, 8 << 20, 16 << 20)
 BLOCK_CANDIDATES = (64, 128, 256)
 # crt_render_params.stage_traversal: CRT_STAGE_LOCAL, _SHARED, _LOCAL_QUANT,
@@ -28,7 +33,7 @@ def cache_key(scene, n_views: int) -> str:
     info = scene.info()
     rp = scene.render_params()
     tris = max(1, int(info["num_triangles"]))
-    return (f"{torch.cuda.get_device_name(scene.ctx.device)}|tris2^{int(math.log2(tris))}|"
+    return (f"v{VERSION}|{torch.cuda.get_device_name(scene.ctx.device)}|tris2^{int(math.log2(tris))}|"
             f"{rp['width']}x{rp['height']}x{n_views}|bounces{rp['max_bounces']}")
 
 
