@@ -55,16 +55,21 @@ def measured_peaks():
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per 16M-ray
 # launch of each trace kernel, from one ncu capture of an 8M-ray launch of
-# the same kernel build on the same batch distribution, scaled x2 (ray bytes
-# scale exactly, node visits linearly for uniform random rays). The capture
-# and its command are summarised in profiles/ (traversal summary).
-TRAFFIC_PER_16M = {"extend": 2 * (564561664 + 132257024), "shadow": 2 * (1538991104 + 26396672)}
+# k_trace_vote on the same batch distribution, scaled x2 (ray bytes scale
+# exactly, node visits linearly for uniform random rays). The capture and its
+# command are summarised in profiles/trace_vote_field_ncu.md.
+TRAFFIC_PER_16M = {"extend": 2 * (555017984 + 143265024), "shadow": 2 * (1377407232 + 61321216)}
 
 
 def profiled_traffic(kernel: str):
     """Per-launch DRAM bytes (16M-ray launch) of `kernel` ("extend" or
     "shadow"), or None if not captured."""
     return TRAFFIC_PER_16M.get(kernel)
+
+
+def without(v, keys):
+    """v with the entries named in `keys` left out of its nested dicts."""
+    return {k: without(w, keys) for k, w in v.items() if k not in keys} if isinstance(v, dict) else v
 
 
 class ClockSampler:
@@ -948,7 +953,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": kern[dom]["achieved"], "peak": peak, "unit": "GB/s",
                          "frac": kern[dom]["frac"], "traffic": kern[dom]["traffic"],
                          "peak_kind": peak_kind,
-                         "kernel": "k_trace_shadow" if dom == "shadow" else "k_trace_closest",
+                         "kernel": "k_trace_vote<ShadowJob>" if dom == "shadow" else "k_trace_vote<ClosestJob>",
                          "algorithmic_bytes_per_launch": kern[dom]["algorithmic_bytes_per_launch"],
                          "bytes_per_unit": SHADOW_BYTES if dom == "shadow" else EXTEND_BYTES},
             "cpu_baseline": cpu,
@@ -964,7 +969,10 @@ def main():
             "gpu_launches": 2 * args.steps,
             "clocks": clocks,
         }
-        print(json.dumps(out))
+        # the legs in full to stderr; the line itself without their tables (per
+        # request class, per layer), which made it 22 KB
+        print(json.dumps({k: v for k, v in out.items() if isinstance(v, dict)}), file=sys.stderr)
+        print(json.dumps(without(out, ("by_class", "layers"))))
     del scene
     ctx.close()
     if world > 1:
