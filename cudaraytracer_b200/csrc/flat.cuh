@@ -4,7 +4,7 @@
 // 32 lanes busy.
 //
 // 1. A conservative test of all triangles from precomputed per-triangle
-//    vectors (18 multiply-adds, no division): with m = o x d,
+//    vectors (22 multiply-adds, no division): with m = o x d,
 //      det = d . (e2 x e1)          T = v0 . (e2 x e1) - o . (e2 x e1)
 //      U = e2 . m - d . (e2 x v0)   V = d . (e1 x v0) - e1 . m
 //    are the numerators of the triangle test (t = T / det, b1 = U / det,
@@ -28,7 +28,7 @@
 // For batches of unordered rays (the trace kernels). Measured on the Cornell
 // box (36 triangles), 1M random rays + 1M shadow queries in one pass: 249 us
 // over the tree in shared memory, 201 with the records in global memory, one
-// triangle at a time (load pipe 82% busy), 154 as here. The renderer's
+// triangle at a time (load pipe 82% busy), 155 as here. The renderer's
 // camera and shadow rays run 5-8% slower this way (256 x 256 frame 613 ->
 // 657 us, 16 views 10.3 -> 11.4 ms): neighbouring paths take the tree
 // together, and its boxes cull most of the triangles.
@@ -71,6 +71,10 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
     const float sd = s1n * d1;
     const float md = 2e-6f * d1 * sc.x * sc.x, mt = 2e-6f * s1n * sc.x * sc.x, mu = 2e-6f * sc.x * sd;
     const float mw = 2.f * (mu + md);
+    // Products beyond the floats, or so small that their roundings are not
+    // relative (huge, tiny or non-finite rays; k_flat keeps 1e-10 <= E <= 1e10
+    // and S >= 1e-12, so no margin falls below 1e-40): the tree decides.
+    bool odd = !(md + mt + mu + sd < 1e30f) || !(d1 > 1e-12f);
     const float mx = o.y * d.z - o.z * d.y, my = o.z * d.x - o.x * d.z, mz = o.x * d.y - o.y * d.x;
     const F2 dx = f2(d.x, d.x), dy = f2(d.y, d.y), dz = f2(d.z, d.z);
     const F2 ox = f2(-o.x, -o.x), oy = f2(-o.y, -o.y), oz = f2(-o.z, -o.z);
@@ -100,11 +104,8 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
     hit.t = tmax;
     hit.slot = -1;
     hit.b1 = hit.b2 = 0.f;
-    float best = INFINITY, second = INFINITY, det_b = 1.f;
-    // Products beyond the floats, or so small that their roundings are not
-    // relative (huge, tiny or non-finite rays; k_flat keeps 1e-10 <= E <= 1e10
-    // and S >= 1e-12, so no margin falls below 1e-40): the tree decides.
-    bool odd = !(md + mt + mu + sd < 1e30f) || !(d1 > 1e-12f), clear = false;
+    float best = INFINITY, second = INFINITY, inv_b = 1.f;
+    bool clear = false;
     while (cand[0] | cand[1]) {
         int slot;
         if (cand[0]) {
@@ -133,7 +134,7 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
         if (t < best) {
             second = best;
             best = t;
-            det_b = det;
+            inv_b = inv;
             hit.slot = slot;
             hit.b1 = b1;
             hit.b2 = b2;
@@ -143,8 +144,10 @@ __device__ __forceinline__ Hit closest_hit_flat(const float4 *rec, const BvhView
         }
     }
     if (hit.slot >= 0) {
-        // rounding of t = T / det: T's, det's and the quotient's
-        const float gap = (mt + md * best) / det_b + 2e-6f * best;
+        // rounding of t = T / det in the triangle test: T's and det's, 8 u of
+        // their scales with the edges' own (the margins are 32 u), and more
+        // than the quotient's and the slabs' few ulp
+        const float gap = 0.25f * (mt + md * best) * inv_b + 2e-6f * best;
         if (best > tmax + gap) {  // beyond the caller's bound, clearly: no hit
             hit.slot = -1;
             hit.b1 = hit.b2 = 0.f;
