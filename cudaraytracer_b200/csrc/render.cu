@@ -746,9 +746,10 @@ struct SceneSrc {
     __device__ void add(const PathState &ps) { accumulate(acc, ps.pixel, ps.dc, ps.ic); }
 };
 
-// Compiled for two register budgets. With 3 resident blocks per SM (168
-// registers) a small pass finishes sooner; with 8 (64 registers, as the shade
-// stage) a large one has the warps to cover instruction fetch (Cornell box,
+// Compiled for two register budgets. Bounded at 3 resident blocks per SM it
+// takes 124-126 registers without spills (four blocks fit) and a small pass
+// finishes sooner; with 8 (64 registers, as the shade stage) a large one has
+// the warps to cover instruction fetch (Cornell box,
 // 262,144 / 8,388,608 paths: 610 / 11,205 us with 3, 690 / 10,507 us with 8).
 template <bool kTiny, int kMinBlocks>
 __global__ void __launch_bounds__(kPathBlock, kMinBlocks) k_paths(SceneView s, StepParams sp, int max_bounces,

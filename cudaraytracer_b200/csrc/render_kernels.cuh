@@ -81,9 +81,9 @@ void launch_shadow_stage(const BvhView &bvh, const ShadowView &sh, int *counters
 // The path kernel (path_loop.cuh): every path of queue q (count *n_in) from
 // bounce sp.bounce to its end; raygen has reset counters[kPathCounter].
 // path_start is the bounce from which a pass of n paths in stage-traversal
-// mode `mode` goes to it (INT_MAX: never, as with CRT_PATH_KERNEL=0): a stage costs its slowest warp's
-// latency and three more launches, 17 us with no path left in it and 65 us
-// with a few, so late bounces and small passes belong in one kernel, while
+// mode `mode` goes to it (INT_MAX: never, as with CRT_PATH_KERNEL=0): a stage
+// costs its slowest warp's latency and three more launches, 17 us with no path
+// left in it and 65 us with a few, so late bounces and small passes belong in one kernel, while
 // the first bounces of large passes run better as stages (compaction, full
 // warps, 64-register shade). Measured, us per pass, stages only / path
 // kernel from bounce 0 / 1 / 2, at 65,536, 1,048,576 and 8,388,608 paths:
